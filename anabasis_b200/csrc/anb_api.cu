@@ -420,6 +420,8 @@ PcgArgsT<float> pcg_args32(anb_ctx* c, const float* b, float* x, double atol, do
 // Coarse levels of at most this many rows run as one cluster kernel (ANB_AMG_TAIL_ROWS overrides;
 // 0 launches every level and sweep separately).  The arithmetic is the same either way.
 constexpr int kAmgTailRows = 1024;
+// The same for the smoothed-aggregation hierarchy.
+constexpr int kSaTailRows = 1024;
 // CSR levels of at most this many rows run down sweep + restriction as one kernel
 // (ANB_AMG_FUSED_DOWN_ROWS overrides; 0 = off).  Same values either way.
 constexpr int kAmgFusedDownRows = 65536;
@@ -427,6 +429,136 @@ constexpr int kAmgFusedDownRows = 65536;
 // Grid of the row-parallel kernels: at most this many 256-thread blocks per SM (grid-stride
 // beyond); ANB_BLOCKS_PER_SM overrides.
 constexpr int kBlocksPerSM = 8;
+
+// Lanes per row of a coarse sweep: about four entries a lane, and more where the rows alone would
+// leave the GPU's 300,000 resident threads idle.
+int sa_lanes(long long entries, int rows) {
+  const double avg = rows > 0 ? (double)entries / rows : 1.0;
+  int g = 4;
+  while (g < 32 && (4 * g < avg || (long long)g * rows < 150000)) g *= 2;
+  while (g > 4 && g >= 2 * avg) g /= 2;  // not more lanes than entries
+  return g;
+}
+
+// Smoothed-aggregation hierarchy of the current level-0 matrix: patterns on the host, values level
+// by level on the device (the next level's strong couplings come from them).  Returns false, with
+// nothing kept, when the coarsening stalls above the dense solver's size.
+template <class T>
+bool build_sa(anb_ctx* c, AmgDevT<T>& A, DevArena& ar, T* val0, T* diag0, T* wdinv0, std::vector<double>& hv,
+              std::vector<double>& hd) {
+  // up to 128 rows the dense inverse keeps its matrix in registers without spills (172 us at 116
+  // rows against 573 us at 160)
+  constexpr int kDenseRows = 128;
+  SaMatrix M = sa_fine_matrix(c->L, hv, hd);
+  auto reset = [&](bool ok) {
+    if (ok) return true;
+    CK(cudaStreamSynchronize(c->stream));
+    ar.release();
+    A.nLevels = 0;
+    A.sa = 0;
+    return false;
+  };
+  if (M.n <= 128) return false;  // plain path: no hierarchy, Jacobi
+  int l = 0;
+  AmgLevelDevT<T>* d = &A.lv[0];
+  *d = AmgLevelDevT<T>{};
+  d->n = M.n;
+  d->sliceOff = c->dm.sliceOff;
+  d->col = c->dm.col;
+  d->val = val0;
+  d->diag = diag0;
+  d->wdinv = wdinv0;
+  d->maxW = c->L.maxRowLen;
+  d->x2 = ar.alloc<T>(M.n);
+  while (M.n > kDenseRows || l == 0) {
+    if (l + 1 >= kSaMaxLevels) return reset(false);
+    // Where the next matrix would grow dense (or have a row too long for a block's shared memory),
+    // half the threshold is tried: fewer weak couplings, larger aggregates.
+    double theta = sa_theta(l, M.n, c->L.maxRowLen);
+    SaPattern S;
+    int nc = 0;
+    AmgLevelDevT<T>& f = A.lv[l];
+    for (int tries = 0;; ++tries, theta *= 0.5) {
+      std::vector<int> agg = sa_aggregate(M, theta, nc);
+      if (nc < 1 || nc > (int)(0.9 * M.n)) return reset(false);
+      S = sa_pattern(M, std::move(agg), nc, l > 0);
+      f.capQ = f.capC = 1;
+      for (int i = 0; i < M.n; ++i) f.capQ = std::max(f.capQ, S.qOff[i + 1] - S.qOff[i]);
+      for (int I = 0; I < nc; ++I) f.capC = std::max(f.capC, S.cOff[I + 1] - S.cOff[I] + 1);
+      const bool fits = sa_product_smem(8, 256, std::max(f.capQ, f.capC)) <= kSaSmemMax;
+      if (fits && (S.cCol.size() <= M.col.size() * 5 / 4 || tries == 3)) break;
+      if (tries == 3) return reset(false);
+    }
+    AmgLevelDevT<T>& k = A.lv[l + 1];
+    k = AmgLevelDevT<T>{};
+    f.nc = nc;
+    f.agg = ar.upload(S.agg);
+    f.pOff = ar.upload(S.pOff);
+    f.pCol = ar.upload(S.pCol);
+    f.pVal = ar.alloc<T>(S.pCol.size());
+    f.qOff = ar.upload(S.qOff);
+    f.qCol = ar.upload(S.qCol);
+    f.apVal = ar.alloc<T>(S.qCol.size());
+    f.ptOff = ar.upload(S.ptOff);
+    f.ptCol = ar.upload(S.ptCol);
+    f.ptSrc = ar.upload(S.ptSrc);
+    if (l == 0) {  // Q in SELL-32 (columns padded with 0, never read)
+      const int nSl = (M.n + kSlice - 1) / kSlice;
+      std::vector<int> sl(nSl + 1, 0);
+      for (int s = 0; s < nSl; ++s) {
+        int w = 0;
+        for (int i = s * kSlice; i < std::min(M.n, (s + 1) * kSlice); ++i) w = std::max(w, S.qOff[i + 1] - S.qOff[i]);
+        sl[s + 1] = sl[s] + w * kSlice;
+      }
+      std::vector<int> cs(sl[nSl], 0);
+#pragma omp parallel for schedule(static)
+      for (int i = 0; i < M.n; ++i)
+        for (int e = S.qOff[i]; e < S.qOff[i + 1]; ++e)
+          cs[sl[i / kSlice] + (e - S.qOff[i]) * kSlice + i % kSlice] = S.qCol[e];
+      f.qSlice = ar.upload(sl);
+      f.qColS = ar.upload(cs);
+      f.qVal = ar.alloc<T>(cs.size());
+      f.tOff = f.ptOff;
+      f.tCol = f.ptCol;
+      f.tSrc = f.ptSrc;
+      f.nT = (int)S.ptCol.size();
+    } else {
+      f.qVal = ar.alloc<T>(S.qCol.size());
+      f.tOff = ar.upload(S.qtOff);
+      f.tCol = ar.upload(S.qtCol);
+      f.tSrc = ar.upload(S.qtSrc);
+      f.nT = (int)S.qtCol.size();
+      f.lanesUp = sa_lanes((long long)M.col.size() + (long long)S.qCol.size(), M.n);
+    }
+    f.tVal = ar.alloc<T>(f.nT);
+    f.lanesDown = sa_lanes(f.nT, nc);
+    k.n = nc;
+    k.rowOff = ar.upload(S.cOff);
+    k.col = ar.upload(S.cCol);
+    k.val = ar.alloc<T>(S.cCol.size());
+    k.diag = ar.alloc<T>(nc);
+    k.wdinv = ar.alloc<T>(nc);
+    k.b = ar.alloc<T>(nc);
+    k.x = ar.alloc<T>(nc);
+    k.x2 = ar.alloc<T>(nc);
+    sa_refresh_level(c->lc, A, l);
+    std::vector<T> v(S.cCol.size()), dg(nc);
+    CK(cudaMemcpyAsync(v.data(), k.val, v.size() * sizeof(T), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(dg.data(), k.diag, dg.size() * sizeof(T), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    M.n = nc;
+    M.off = S.cOff;
+    M.col = S.cCol;
+    M.val.assign(v.begin(), v.end());
+    M.diag.assign(dg.begin(), dg.end());
+    ++l;
+  }
+  A.nLevels = l + 1;
+  A.sa = 1;
+  A.nDense = M.n;
+  A.dense = ar.alloc<double>((size_t)M.n * M.n);
+  return true;
+}
 
 // Aggregation hierarchy for the current level-0 matrix (val0/diag0 on the device, storage type T),
 // coarse levels in T, coarsest inverse in double, host structure in H, device arrays in ar.  For the
@@ -438,6 +570,16 @@ void build_amg(anb_ctx* c, AmgDevT<T>& A, std::vector<AmgLevelHost>& H, DevArena
   CK(cudaMemcpyAsync(hv.data(), val0, hv.size() * sizeof(T), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaMemcpyAsync(hd.data(), diag0, hd.size() * sizeof(T), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
+  std::vector<double> hvd(hv.begin(), hv.end()), hdd(hd.begin(), hd.end());
+  const char* noGraph = std::getenv("ANB_NO_GRAPH");
+  if (ga && build_sa(c, A, ar, val0, diag0, wdinv0, hvd, hdd)) {
+    H.clear();
+    c->amgBuilt = true;
+    sa_configure_tail(A, kSaTailRows, c->stream);
+    if (!(noGraph && noGraph[0] == '1')) CK(amg_capture_graph(c->lc, *ga, A));
+    return;
+  }
+  A.sa = 0;
   AmgSetupOptions opt;
   if (const char* sr = std::getenv("ANB_AMG_SELL_MIN_ROWS")) opt.sellMinRows = std::atoi(sr);
   if (const char* ps = std::getenv("ANB_AMG_PASSES")) {  // e.g. "2,2,3": passes per level
@@ -447,8 +589,7 @@ void build_amg(anb_ctx* c, AmgDevT<T>& A, std::vector<AmgLevelHost>& H, DevArena
       if (*q == ',') ++q;
     }
   }
-  H = build_amg_hierarchy(c->L, std::vector<double>(hv.begin(), hv.end()),
-                                   std::vector<double>(hd.begin(), hd.end()), opt);
+  H = build_amg_hierarchy(c->L, hvd, hdd, opt);
   A.nLevels = (int)H.size();
   for (int l = 0; l < A.nLevels; ++l) {
     const AmgLevelHost& h = H[l];
@@ -512,7 +653,6 @@ void build_amg(anb_ctx* c, AmgDevT<T>& A, std::vector<AmgLevelHost>& H, DevArena
                    l == 0 ? c->L.maxRowLen : H[l].maxW);
     std::fprintf(stderr, " | tail rows %d, cluster %d\n", A.tailRows, A.tailCluster);
   }
-  const char* noGraph = std::getenv("ANB_NO_GRAPH");
   if (ga && A.nLevels >= 2 && !(noGraph && noGraph[0] == '1')) CK(amg_capture_graph(c->lc, *ga, A));
 }
 
@@ -924,10 +1064,10 @@ void build_slot_lookup(anb_ctx* c) {
 void release_amg(anb_ctx* c) {
   CK(cudaStreamSynchronize(c->stream));
   amg_release_graphs(c->amg);
-  c->amg.nLevels = 0;
+  c->amg.nLevels = c->amg.sa = 0;
   c->amg.dense = nullptr;
   amg_release_graphs(c->amg32);
-  c->amg32.nLevels = 0;
+  c->amg32.nLevels = c->amg32.sa = 0;
   c->amg32.dense = nullptr;
   c->amgArena.release();
   c->amgHost.clear();

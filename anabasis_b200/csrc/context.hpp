@@ -15,6 +15,7 @@
 #include "host_mesh.hpp"
 #include "kernels.cuh"
 #include "layout.hpp"
+#include "sa_setup.hpp"
 
 namespace anb {
 

@@ -331,6 +331,15 @@ struct AmgLevelDevT {
   T *b, *x, *x2;
   T* wdinv;            // omega / diag (Jacobi smoother)
   int maxW;            // level 0: largest SELL slice width
+  // smoothed-aggregation hierarchies (AmgDevT::sa) only.  P by rows; A P by rows (the pattern of Q) and
+  // Q = (I - w D^-1 A) P, whose values on level 0 are SELL-32 (qSlice, qColS: thread per row) and
+  // elsewhere follow qCol; the restriction operator by coarse rows, gathered from pVal (level 0: P^T)
+  // or qVal (Q^T); P^T for the Galerkin product.
+  const int *pOff, *pCol, *qOff, *qCol, *qSlice, *qColS, *tOff, *tCol, *tSrc, *ptOff, *ptCol, *ptSrc;
+  T *pVal, *apVal, *qVal, *tVal;
+  int nT;              // entries of the restriction operator
+  int lanesDown, lanesUp;  // lanes per row of the restriction from and the up sweep of this level
+  int capQ, capC;      // longest row of Q, and of the next level's matrix + 1
 };
 template <class T>
 struct AmgDevT {
@@ -359,6 +368,8 @@ struct AmgDevT {
   // CSR levels of at most this many rows (above the tail) run their down sweep and restriction
   // as one kernel, warp per aggregate (same values; fewer launches, longer chains per warp)
   int fusedDownRows = 0;
+  // 1: smoothed aggregation (kernels_sa.cu), 0: plain aggregation with over-correction
+  int sa = 0;
 };
 using AmgLevelDev = AmgLevelDevT<double>;
 using AmgDev = AmgDevT<double>;
@@ -373,6 +384,27 @@ template <class T>
 void pcg_precondition(const LaunchCfg& lc, const PcgArgsT<T>& a, const AmgDevT<T>* amg);
 template <class T>
 void amg_refresh(const LaunchCfg& lc, AmgDevT<T>& amg);  // Galerkin values + dense inverse
+// Inverse of the matrix of a CSR level of at most 160 rows (the coarsest) into inv.
+template <class T>
+void amg_dense_factor(const LaunchCfg& lc, const AmgLevelDevT<T>& c, double* inv);
+// Smoothed-aggregation counterparts (kernels_sa.cu): values of one level step (P, Q, restriction and
+// the next level's matrix), all of them with the dense inverse, and the V-cycle of the PCG (mode 0).
+constexpr double kSaOmegaP = 2.0 / 3.0;
+template <class T>
+void sa_refresh_level(const LaunchCfg& lc, AmgDevT<T>& amg, int l);
+template <class T>
+void sa_refresh(const LaunchCfg& lc, AmgDevT<T>& amg);
+// Dynamic shared memory of one block of the refresh's sparse products, and whether a row of the product
+// goes to one warp (many rows) or to a whole block.
+constexpr size_t kSaSmemMax = 200 * 1024;
+inline size_t sa_product_smem(int G, int TS, int cap) {
+  return (size_t)(kBlock / TS) * cap * ((size_t)(TS / G) * sizeof(double) + sizeof(int));
+}
+inline bool sa_small_team(int rows, int cap) { return rows >= 16384 && sa_product_smem(4, 32, cap) <= kSaSmemMax; }
+template <class T>
+void sa_configure_tail(AmgDevT<T>& amg, int tailRows, cudaStream_t s);
+template <class T>
+void sa_vcycle(const LaunchCfg& lc, const PcgArgsT<T>& a, const AmgDevT<T>* amg, int v);
 // z = M^-1 r with one V-cycle for arguments in mode 1 (r input, r2 scratch, z output, fl[0] a done
 // flag that skips the application); captured into *graph on the first call when graph != nullptr
 template <class T>

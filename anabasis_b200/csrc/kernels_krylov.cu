@@ -17,17 +17,12 @@
 
 #include <cooperative_groups.h>
 
-#include "kernels.cuh"
+#include "krylov_dev.cuh"
 
 namespace anb {
 namespace {
 
 namespace cg = cooperative_groups;
-
-template <class T>
-__device__ __forceinline__ double ld(const T* p) {
-  return (double)__ldg(p);
-}
 
 // y = (D + Off) x for one row of a SELL-32 matrix
 template <class T, class X>
@@ -62,28 +57,6 @@ __device__ __forceinline__ void sell_row3(const DSellT<T>& A, int r, const T* x,
 #pragma unroll
     for (int c = 0; c < 3; ++c)
       if (c < nc && act[c]) y[c] += v * (double)x[c * n + j];
-  }
-}
-
-// Row r's slots in registers, for a compile-time bound WM on the slice width: every column and
-// value load of the row is issued before the first gather, so a row costs two dependent memory
-// round trips instead of two per unrolled group.  Slots past the row's slice width are
-// (column r, value 0) and read nothing.
-template <int WM, class T>
-__device__ __forceinline__ void sell_regs(const int* sliceOff, const int* col, const T* val, int r, int (&c)[WM],
-                                          double (&v)[WM]) {
-  const int s = r >> 5;
-  const int b0 = __ldg(&sliceOff[s]);
-  const int W = (__ldg(&sliceOff[s + 1]) - b0) >> 5;
-  const int b = b0 + (r & 31);
-#pragma unroll
-  for (int k = 0; k < WM; ++k) {
-    c[k] = r;
-    v[k] = 0.0;
-    if (k < W) {
-      c[k] = __ldg(&col[b + (k << 5)]);
-      v[k] = ld(&val[b + (k << 5)]);
-    }
   }
 }
 
@@ -471,20 +444,6 @@ __global__ void __launch_bounds__(kBlock) k_pcg_pq(PcgArgsT<T> a, const T* pOld,
   }
 }
 
-// Iteration count and convergence test on |r|^2 = rr (last block, thread 0).
-template <class T>
-__device__ __forceinline__ void pcg_converged(const PcgArgsT<T>& a, double rr) {
-  a.sc[4] = rr;
-  a.fl[1] += 1;
-  if (sqrt(rr) <= a.sc[3]) {
-    a.fl[0] = 1;
-    a.fl[2] = 1;
-  } else if (a.fl[1] >= a.maxit || a.sc[5] == 0.0) {
-    a.fl[0] = 1;
-    a.fl[2] = 0;
-  }
-}
-
 // x += alpha p ; r -= alpha q ; convergence test on |r|
 template <class T>
 __global__ void __launch_bounds__(kBlock) k_pcg_xr(PcgArgsT<T> a, const T* p) {
@@ -619,13 +578,6 @@ struct LdL2 {
 // so splitting rows keeps enough loads in flight.  The warp-level loop bound keeps every lane of
 // a warp in the shuffles.  The row sweeps are device functions over (warp, nWarps) so that the
 // per-level kernels and the cluster tail run the same arithmetic.
-template <int G>
-__device__ __forceinline__ double group_sum(double v) {
-#pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o, G);
-  return v;
-}
-
 // Down, part 1 on a CSR level: x = w D^-1 b, x2 = b - A x.
 template <int G, class T, class LD>
 __device__ __forceinline__ void resid_csr_rows(const AmgLevelDevT<T>& f, int warp, int nWarps, LD ldv) {
@@ -1157,6 +1109,7 @@ void amg_configure_tail(AmgDevT<T>& amg, int tailRows, cudaStream_t s) {
 // the other and updates x with p_v.
 template <class T>
 static void vcycle(const LaunchCfg& lc, const PcgArgsT<T>& a, const AmgDevT<T>* amg, int v) {
+  if (amg->sa) return sa_vcycle(lc, a, amg, v);
   const int L = amg->nLevels;
   const T* rIn = v ? a.r2 : a.r;
   T* rOut = v ? a.r : a.r2;
@@ -1473,8 +1426,27 @@ void amg_apply(const LaunchCfg& lc, const PcgArgsT<T>& a, const AmgDevT<T>* amg,
   }
 }
 
+// Inverse of the coarsest matrix (CSR, at most kDenseMax rows) into inv.
+template <class T>
+void amg_dense_factor(const LaunchCfg& lc, const AmgLevelDevT<T>& c, double* inv) {
+  const size_t smem = sizeof(double) * (size_t)c.n * c.n;
+  g_launches += 1;
+  const int nc = (c.n + 31) / 32;
+  auto go = [&](auto kern) {
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    kern<<<1, 1024, smem, lc.stream>>>(c, inv);
+  };
+  if (nc <= 1) go(k_amg_dense_factor<T, 1>);
+  else if (nc == 2) go(k_amg_dense_factor<T, 2>);
+  else if (nc == 3) go(k_amg_dense_factor<T, 3>);
+  else if (nc == 4) go(k_amg_dense_factor<T, 4>);
+  else go(k_amg_dense_factor<T, 5>);
+}
+
+
 template <class T>
 void amg_refresh(const LaunchCfg& lc, AmgDevT<T>& amg) {
+  if (amg.sa) return sa_refresh(lc, amg);
   for (int l = 0; l + 1 < amg.nLevels; ++l) {
     AmgLevelDevT<T>& f = amg.lv[l];
     AmgLevelDevT<T>& c = amg.lv[l + 1];
@@ -1482,19 +1454,7 @@ void amg_refresh(const LaunchCfg& lc, AmgDevT<T>& amg) {
     k_amg_galerkin<T><<<blocks_for(f.nEntNext + f.nc, lc.rowBlocks), kBlock, 0, lc.stream>>>(f, c.val, c.diag,
                                                                                              c.wdinv, amg.omega);
   }
-  const AmgLevelDevT<T>& c = amg.lv[amg.nLevels - 1];
-  const size_t smem = sizeof(double) * (size_t)c.n * c.n;
-  g_launches += 1;
-  const int nc = (c.n + 31) / 32;
-  auto go = [&](auto kern) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    kern<<<1, 1024, smem, lc.stream>>>(c, amg.dense);
-  };
-  if (nc <= 1) go(k_amg_dense_factor<T, 1>);
-  else if (nc == 2) go(k_amg_dense_factor<T, 2>);
-  else if (nc == 3) go(k_amg_dense_factor<T, 3>);
-  else if (nc == 4) go(k_amg_dense_factor<T, 4>);
-  else go(k_amg_dense_factor<T, 5>);
+  amg_dense_factor(lc, amg.lv[amg.nLevels - 1], amg.dense);
 }
 
 void launch_defect(const LaunchCfg& lc, const DefectArgs& a) {
@@ -1519,6 +1479,7 @@ void launch_apply_correction(const LaunchCfg& lc, int n, int nc, double* x, floa
   template void pcg_iteration<T>(const LaunchCfg&, const PcgArgsT<T>&, int, const AmgDevT<T>*); \
   template void pcg_precondition<T>(const LaunchCfg&, const PcgArgsT<T>&, const AmgDevT<T>*);  \
   template void amg_refresh<T>(const LaunchCfg&, AmgDevT<T>&);                                \
+  template void amg_dense_factor<T>(const LaunchCfg&, const AmgLevelDevT<T>&, double*);        \
   template cudaError_t amg_capture_graph<T>(const LaunchCfg&, const PcgArgsT<T>&, AmgDevT<T>&);           \
   template bool pcg_loop_launch<T>(const LaunchCfg&, const PcgArgsT<T>&, const AmgDevT<T>&);  \
   template void amg_release_graphs<T>(AmgDevT<T>&);                                           \

@@ -1,0 +1,53 @@
+// Host structure set-up of the smoothed-aggregation hierarchy that preconditions the pressure CG.
+//
+// One level step: strong couplings (a_ij < 0, a_ij^2 > theta^2 a_ii a_jj) give star aggregates (a
+// root with all its strong neighbours where all of them are free; the rows left over join the
+// aggregate of their strongest aggregated neighbour, what remains forms aggregates of its own).  The
+// prolongator is P = (I - omegaP D^-1 A) P0 with P0 piecewise constant.  Only patterns are made here:
+// they follow the matrix pattern and the aggregates, never the values, so the device can refresh every
+// value in place when the matrix changes (sa_refresh).
+#pragma once
+
+#include <vector>
+
+#include "layout.hpp"
+
+namespace anb {
+
+// Off-diagonal CSR with the diagonal apart.
+struct SaMatrix {
+  int n = 0;
+  std::vector<int> off, col;
+  std::vector<double> val, diag;
+};
+
+struct SaPattern {
+  int n = 0, nc = 0;
+  std::vector<int> agg;                 // n
+  std::vector<int> pOff, pCol;          // P by rows: the aggregates of the row and its neighbours
+  std::vector<int> qOff, qCol;          // A P by rows (the pattern of P is part of it)
+  std::vector<int> ptOff, ptCol, ptSrc; // P^T by rows: fine row and entry of P
+  std::vector<int> qtOff, qtCol, qtSrc; // Q^T by rows: fine row and entry of Q (only on request)
+  std::vector<int> cOff, cCol;          // off-diagonals of the next level's matrix P^T A P
+};
+
+constexpr int kSaMaxLevels = 12;
+// Threshold of the strong couplings.  On the finest level 0.02 keeps every face of a mildly stretched
+// hex grid strong (level 1: n / 8 rows of 30 entries), 0.1 coarsens along the strong directions only
+// (n / 5.6 rows of 38): fewer iterations of a dearer cycle, which pays where launches and not bytes
+// set the cycle's time (ms per SIMPLE step, 0.1 / 0.02: 16k hexes 2.00 / 2.24, 36k 5.5 / 6.1, 250k
+// 6.3 / 5.65, 970k 20.4 / 18.4) and on tetrahedra, whose rows stay short (334k 9.7 / 10.3).  Below,
+// 0.04 (0.02: 82 iterations a step at 970k cells instead of 65; 0.06: matrices too dense).
+inline double sa_theta(int level, int n, int maxRowLen) {
+  if (level > 0) return 0.04;
+  return n <= 100000 || maxRowLen <= 4 ? 0.1 : 0.02;
+}
+
+// Aggregate of every row; nc receives the count.  Aggregates are numbered by their first row.
+std::vector<int> sa_aggregate(const SaMatrix& A, double theta, int& nc);
+// All patterns of one level step for the given aggregates.
+SaPattern sa_pattern(const SaMatrix& A, std::vector<int> agg, int nc, bool wantQT);
+// The level-0 matrix as CSR; vals in the layout's SELL-32 storage.
+SaMatrix sa_fine_matrix(const Layout& L, const std::vector<double>& vals, const std::vector<double>& diag);
+
+}  // namespace anb
