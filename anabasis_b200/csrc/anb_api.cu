@@ -1367,7 +1367,6 @@ int anb_create(const anb_mesh_desc* md, const anb_params* prm, anb_ctx** out) {
     c->scal = A.alloc<double>(64);
     c->flags = A.alloc<int>(kFlagCount);
     c->stats = A.alloc<double>(16);
-    c->forceOut = A.alloc<double>(16);
     c->red.partials = A.alloc<double>((size_t)(c->lc.rowBlocks + 16) * 16);
     c->red.ticket = A.alloc<unsigned int>(1);
     CK(cudaMemset(c->red.ticket, 0, sizeof(unsigned int)));
@@ -1539,9 +1538,9 @@ int anb_patch_force(anb_ctx* c, int patch, int sign, anb_force_report* out) {
     CK(cudaSetDevice(c->prm.device));
     const int b0 = c->hm.patches[patch].start - c->nI;
     const int b1 = b0 + c->hm.patches[patch].nFaces;
-    launch_patch_force(c->stream, c->dm, b0, b1, sign, c->prm.mu, c->dBA, c->dBN, c->U, c->P, c->forceOut);
-    double h[16];
-    CK(cudaMemcpyAsync(h, c->forceOut, sizeof(double) * 15, cudaMemcpyDeviceToHost, c->stream));
+    double* h = c->hScal + kHostForce;  // pinned: the kernel writes its results here itself
+    launch_patch_force(c->lc, c->dm, b0, b1, sign, c->prm.mu, c->dBA, c->dBN, c->U, c->P, c->red, h);
+    CK(cudaGetLastError());
     CK(cudaStreamSynchronize(c->stream));
     out->valid = 1;
     for (int k = 0; k < 3; ++k) {

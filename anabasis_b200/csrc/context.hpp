@@ -103,7 +103,6 @@ struct anb_ctx {
   double* scal = nullptr;     // device scalars
   int* flags = nullptr;
   double* stats = nullptr;
-  double* forceOut = nullptr;
   Reducer red{};
   // pinned host mirrors
   int* hFlags = nullptr;
@@ -171,6 +170,7 @@ constexpr int kFlagPcg = 32;    // 8: done, iterations, converged, first, loop-g
 constexpr int kFlagCount = 40;  // ints in anb_ctx::flags (and hFlags)
 constexpr int kDeferSlots = 64;
 constexpr int kDeferInts = 16;
+constexpr int kHostForce = 48;  // 15 doubles of anb_ctx::hScal: patch-force results
 constexpr int kScalRelchg = 56; // 6: momentum relative-change sums
 
 int fail(anb_ctx* c, const AnbError& e);

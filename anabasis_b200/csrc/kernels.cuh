@@ -242,8 +242,8 @@ void launch_relchg3(const LaunchCfg& lc, int n, const double* before, const doub
 
 // Patch force (compute_patch_forces_wall_shear, main.cu:2828-2933) over boundary faces
 // [b0, b1); out: Fp[3] Fv[3] F[3] area nFaces minDn maxDn maxUt maxShear (15 doubles).
-void launch_patch_force(cudaStream_t s, const DMesh& m, int b0, int b1, int sign, double mu,
-                        const double* bA, const double* bN, const double* U, const double* P, double* out);
+void launch_patch_force(const LaunchCfg& lc, const DMesh& m, int b0, int b1, int sign, double mu, const double* bA,
+                        const double* bN, const double* U, const double* P, Reducer red, double* out);
 
 // ---- Krylov ----------------------------------------------------------------------------
 // T is the storage type of the matrix values and the solver vectors (double: plain method,

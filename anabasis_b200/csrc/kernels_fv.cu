@@ -5,6 +5,7 @@
 // faces, and accumulates diagonal, right-hand side and divergence in registers.  Each row writes
 // only its own outputs, so the reference's FP64 atomicAdd scatters (main.cu:56-58) become
 // deterministic gathers; a face's flux is written by its owner row.
+#include <algorithm>
 #include <cstdlib>
 #include <mutex>
 #include <string>
@@ -585,9 +586,16 @@ __global__ void __launch_bounds__(kBlock) k_flux_cells(DMesh m, FluxArgs a) {
     for (int q = 0; q < 9; ++q) a.stats[q] = acc[q];
 }
 
-// ---- patch force: main.cu:2828-2933 (single block, deterministic order) -------------------
-__global__ void k_patch_force(DMesh m, int b0, int b1, int sign, double mu, const double* bA, const double* bN,
-                              const double* U, const double* P, double* out) {
+// ---- patch force: main.cu:2828-2933 (deterministic order) ---------------------------------
+// A face's loads are two dependent round trips and nothing else bounds the kernel, so a patch gets a
+// face a thread: one block up to kForceOneBlock faces (no combination across blocks: 31.8 -> 19 us a
+// call for 384 faces), beyond it 256-thread blocks up to a full wave with the last block combining the
+// partials (55,160 wall faces: 252 us a call with one block of 512 threads, 25 us now).  out may be
+// pinned host memory: the 15 results need no copy of their own.
+constexpr int kForceOneBlock = 512;
+__global__ void __launch_bounds__(kForceOneBlock) k_patch_force(DMesh m, int b0, int b1, int sign, double mu,
+                                                                const double* bA, const double* bN, const double* U,
+                                                                const double* P, Reducer red, double* out) {
   __shared__ double sm[16 * 32];
   const int C = m.nCells;
   double v[16];
@@ -596,7 +604,7 @@ __global__ void k_patch_force(DMesh m, int b0, int b1, int sign, double mu, cons
   v[12] = -1.0e308;  // max dn
   v[13] = -1.0e308;  // max |Ut|
   v[14] = -1.0e308;  // max shear
-  for (int b = b0 + threadIdx.x; b < b1; b += blockDim.x) {
+  for (int b = b0 + blockIdx.x * blockDim.x + threadIdx.x; b < b1; b += gridDim.x * blockDim.x) {
     const int r = m.bOwner[b];
     const double A = bA[b];
     if (A <= 1.0e-300) continue;
@@ -631,7 +639,9 @@ __global__ void k_patch_force(DMesh m, int b0, int b1, int sign, double mu, cons
     v[13] = fmax(v[13], Ut);
     v[14] = fmax(v[14], mu * Ut / dn);
   }
-  block_reduce<16>(v, (1u << 11) | (1u << 12) | (1u << 13) | (1u << 14), sm);
+  constexpr unsigned kMax = (1u << 11) | (1u << 12) | (1u << 13) | (1u << 14);
+  if (gridDim.x == 1) block_reduce<16>(v, kMax, sm);
+  else if (!grid_reduce<16>(v, kMax, red, sm)) return;
   if (threadIdx.x == 0) {
     for (int q = 0; q < 11; ++q) out[q] = v[q];
     out[11] = v[10] > 0 ? -v[11] : 0.0;
@@ -798,10 +808,16 @@ void launch_flux_final(const LaunchCfg& lc, const DMesh& m, const FluxArgs& a) {
   else if (wc == 6 || wc == 8) launch_rows(lc, lc.rowBlocks, k_flux_final<8>, m, a);
   else launch_rows(lc, lc.rowBlocks, k_flux_final<0>, m, a);
 }
-void launch_patch_force(cudaStream_t s, const DMesh& m, int b0, int b1, int sign, double mu, const double* bA,
-                        const double* bN, const double* U, const double* P, double* out) {
+void launch_patch_force(const LaunchCfg& lc, const DMesh& m, int b0, int b1, int sign, double mu, const double* bA,
+                        const double* bN, const double* U, const double* P, Reducer red, double* out) {
   g_launches += 1;
-  k_patch_force<<<1, 512, 0, s>>>(m, b0, b1, sign, mu, bA, bN, U, P, out);
+  const int n = b1 - b0;
+  if (n <= kForceOneBlock) {
+    k_patch_force<<<1, std::max(32, (n + 31) / 32 * 32), 0, lc.stream>>>(m, b0, b1, sign, mu, bA, bN, U, P, red, out);
+    return;
+  }
+  const int blocks = std::min(lc.rowBlocks, (n + kBlock - 1) / kBlock);
+  k_patch_force<<<blocks, kBlock, 0, lc.stream>>>(m, b0, b1, sign, mu, bA, bN, U, P, red, out);
 }
 
 }  // namespace anb
