@@ -232,6 +232,12 @@ void mom_solve(anb_ctx* c, AdjointData& d, bool trans, const double* b, double* 
   a.maxit = d.momMaxit;
   a.red = c->red;
   CK(cudaMemsetAsync(x, 0, sizeof(double) * 3 * c->C, c->stream));
+  if (bicg_coop_solve(c->lc, a, 7, c->nSM, c->coopPart)) {
+    poll(c, a.fl, 14);
+    check_coop(c->hFlags);
+    d.momIts += std::max(c->hFlags[2], std::max(c->hFlags[6], c->hFlags[10]));
+    return;
+  }
   bicg_init(c->lc, a);
   int done = 0;
   while (true) {

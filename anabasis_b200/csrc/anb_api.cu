@@ -161,6 +161,10 @@ void poll(anb_ctx* c, const int* dflags, int count) {
   CK(cudaStreamSynchronize(c->stream));
 }
 
+void check_coop(const int* flags) {
+  if (flags[13]) throw AnbError(ANB_ERR_CUDA, "a grid barrier of the BiCGSTAB kernel timed out");
+}
+
 // Outcome of one linear solve: iterations and convergence per component, or, for a solve that ran
 // as a loop graph with its read-back deferred, the hDefer slot its flags arrive in once the stream
 // has synchronised (resolve_solve).
@@ -172,6 +176,7 @@ struct SolveOut {
   int its[3] = {0, 0, 0};
   bool conv[3] = {true, true, true};
   long long kernelsPerIteration = 0;  // loop-graph launch bookkeeping
+  bool coop = false;                  // one cooperative kernel (bicg_coop_solve)
 };
 
 // Queues the copy of a loop-graph solve's flags into the next hDefer slot; with every slot taken it
@@ -195,6 +200,7 @@ void resolve_solve(anb_ctx* c, SolveOut& o) {
   o.resolved = true;
   const int* f = o.slot >= 0 ? c->hDefer + o.slot * kDeferInts : c->hFlags;
   if (o.momentum) {
+    if (o.coop) check_coop(f);
     int mx = 0;
     for (int q = 0; q < 3; ++q) {
       o.its[q] = o.active[q] ? f[4 * q + 2] : 0;
@@ -288,6 +294,15 @@ void solve_momentum(anb_ctx* c, const int* active, SolveOut* out, bool defer) {
   a.maxit = c->prm.vel_maxit;
   a.red = c->red;
   a.precond = (c->prm.mom_amg && c->momAmgBuilt && c->amgMom.nLevels >= 2) ? 1 : 0;
+  const int fam = c->prof.family;
+  if (fam != kKfBicgSpmv && fam != kKfBicgVector &&
+      bicg_coop_solve(c->lc, a, active[0] | active[1] << 1 | active[2] << 2, c->nSM, c->coopPart)) {
+    out->coop = true;
+    if (defer) out->slot = defer_flags(c, a.fl, 14);
+    else poll(c, a.fl, 14);
+    if (!(defer && out->slot >= 0)) resolve_solve(c, *out);
+    return;
+  }
   bicg_init(c->lc, a);
   // freeze inactive components
   for (int q = 0; q < 3; ++q)
@@ -1368,6 +1383,8 @@ int anb_create(const anb_mesh_desc* md, const anb_params* prm, anb_ctx** out) {
     c->flags = A.alloc<int>(kFlagCount);
     c->stats = A.alloc<double>(16);
     c->red.partials = A.alloc<double>((size_t)(c->lc.rowBlocks + 16) * 16);
+    c->nSM = nSM;
+    if (!c->mixed) c->coopPart = A.alloc<double>(bicg_coop_partials(nSM));
     c->red.ticket = A.alloc<unsigned int>(1);
     CK(cudaMemset(c->red.ticket, 0, sizeof(unsigned int)));
     if (!c->mixed) {
@@ -1769,8 +1786,15 @@ int anb_scalar_transport_solve(anb_ctx* c, const double* flux, const double* gam
     for (int outer = 0; outer < nOuter; ++outer) {
       if (a.nonorth) launch_scalar_grad(c->lc, c->dm, a);
       launch_scalar_assemble(c->lc, c->dm, a);
-      bicg_init(c->lc, b);
       int done = 0;
+      if (bicg_coop_solve(c->lc, b, 1, c->nSM, c->coopPart)) {
+        poll(c, b.fl, 14);
+        check_coop(c->hFlags);
+        its = c->hFlags[2];
+        allConv = allConv && c->hFlags[3] != 0;
+        continue;
+      }
+      bicg_init(c->lc, b);
       while (true) {
         for (int k = 0; k < 16; ++k) bicg_iteration(c->lc, b);
         done += 16;

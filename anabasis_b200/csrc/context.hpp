@@ -104,6 +104,8 @@ struct anb_ctx {
   int* flags = nullptr;
   double* stats = nullptr;
   Reducer red{};
+  double* coopPart = nullptr;  // block partials of bicg_coop_solve
+  int nSM = 0;
   // pinned host mirrors
   int* hFlags = nullptr;
   // flags of the solves that ran as loop graphs in the current step, copied here asynchronously
@@ -216,6 +218,8 @@ DSell mom_sell(const anb_ctx* c);
 DSell p_sell(const anb_ctx* c);
 void grad(anb_ctx* c, int nf, const double* const* phi, const unsigned char* bits, double* const* out);
 void poll(anb_ctx* c, const int* dflags, int count);
+// Throws when the flags of a BiCGSTAB solve report a barrier that timed out (bicg_coop_solve).
+void check_coop(const int* flags);
 PcgArgs pcg_args(anb_ctx* c, const double* b, double rtol);
 void solve_pressure(anb_ctx* c, const double* b, double* x, double rtol, int* its, bool* conv);
 void ensure_amg(anb_ctx* c);

@@ -285,6 +285,16 @@ bool bicg_loop_launch(const LaunchCfg& lc, const BicgArgsT<T>& a, BicgLoopT<T>& 
 template <class T>
 void bicg_loop_release(BicgLoopT<T>& loop);
 
+// A whole FP64 Jacobi-BiCGSTAB solve (init included) as one cooperative kernel, for systems of at most
+// kCoopRows rows per thread and component of one 512-thread block per SM (kernels_bicg_coop.cu).
+// Components without their bit in mask are left alone (done, converged, 0 iterations).  partials:
+// bicg_coop_partials(nSM) doubles.  Results as bicg_iteration's, and fl[13] != 0 after a barrier that
+// timed out.  False: nothing was launched.
+constexpr int kCoopRows = 4;
+int bicg_coop_partials(int nSM);
+bool bicg_coop_fits(int n, int nc, int nSM);
+bool bicg_coop_solve(const LaunchCfg& lc, const BicgArgs& a, int mask, int nSM, double* partials);
+
 template <class T>
 struct PcgArgsT {
   DSellT<T> A;
