@@ -1591,21 +1591,30 @@ void ensure_scalar_buffers(anb_ctx* c) {
   c->sSp = A.alloc<double>(C);
   c->sPhi = A.alloc<double>(C);
   c->sGrad = A.alloc<double>((size_t)3 * C);
+  c->sRaw = A.alloc<double>(nF);
+  c->sOrig = A.upload(c->L.fOrig);
+  c->sFlip = A.upload(c->L.fFlip);
 }
 
 // Face array in input order/orientation -> device (layout order; fluxes change sign on flipped
 // internal faces).  src == nullptr uploads `fill`.
 void upload_faces(anb_ctx* c, const double* src, double* dst, bool orientSign, double fill) {
   const int nF = c->nI + c->nB;
-  std::vector<double> h(nF, fill);
-  if (src) {
-    for (int fi = 0; fi < c->nI; ++fi) {
-      const double v = src[c->L.fOrig[fi]];
-      h[fi] = (orientSign && c->L.fFlip[fi]) ? -v : v;
-    }
-    for (int b = 0; b < c->nB; ++b) h[c->nI + b] = src[c->nI + b];
+  if (!src) {
+    launch_fill(c->lc, nF, fill, dst);
+    return;
   }
-  CK(cudaMemcpyAsync(dst, h.data(), nF * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+  // the caller's array goes up as it is, through the pinned buffer in chunks, and is permuted there
+  const size_t cap = (size_t)4 * c->C, ch = stage_chunk(c->C);
+  for (size_t o = 0; o < (size_t)nF;) {
+    const size_t n = std::min(ch, (size_t)nF - o), h = o % cap, m = std::min(n, cap - h);
+    if (o > 0 && h == 0) CK(cudaStreamSynchronize(c->stream));  // the buffer goes round
+    host_copy(c->hStage + h, src + o, m);
+    CK(cudaMemcpyAsync(c->sRaw + o, c->hStage + h, m * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    o += m;
+  }
+  launch_permute_faces(c->lc, c->nI, nF, c->sOrig, c->sFlip, orientSign, c->sRaw, dst);
+  CK(cudaGetLastError());
   CK(cudaStreamSynchronize(c->stream));
 }
 
@@ -1614,15 +1623,13 @@ void upload_cells1(anb_ctx* c, const double* src, double* dst, double fill) {
     const double* s[1] = {src};
     upload_cells(c, s, dst, 1);
   } else {
-    std::vector<double> h(c->C, fill);
-    CK(cudaMemcpyAsync(dst, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    launch_fill(c->lc, c->C, fill, dst);
   }
 }
 
 // Boundary types/values (nFaces arrays, boundary entries read) -> device, LSQ inverse for them.
 void upload_scalar_bc(anb_ctx* c, const int* type, const double* value, int maxType) {
-  std::vector<uint8_t> t(c->nB), dir(c->nB);
+  std::vector<uint8_t> t(c->nB);
   std::vector<double> v(c->nB);
   for (int b = 0; b < c->nB; ++b) {
     const int ty = type[c->nI + b];
@@ -1630,14 +1637,15 @@ void upload_scalar_bc(anb_ctx* c, const int* type, const double* value, int maxT
       throw AnbError(ANB_ERR_INVALID, "invalid scalar boundary type " + std::to_string(ty) + " at face " +
                                           std::to_string(c->nI + b));
     t[b] = (uint8_t)ty;
-    dir[b] = ty == ANB_SCALAR_DIRICHLET;
     v[b] = value[c->nI + b];
   }
-  const std::vector<double> minv = scalar_lsq_minv(c->hm, c->L, dir);
   CK(cudaMemcpyAsync(c->sBcType, t.data(), t.size(), cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(c->sBcVal, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpyAsync(c->sMinv, minv.data(), minv.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+  ScalarArgs a{};
+  a.bcType = c->sBcType;
+  a.bN = c->dBN;
+  launch_scalar_minv(c->lc, c->dm, a, c->sMinv);
+  CK(cudaStreamSynchronize(c->stream));  // t and v go
 }
 
 ScalarArgs scalar_args(anb_ctx* c) {
@@ -1729,12 +1737,7 @@ int anb_scalar_elliptic_solve(anb_ctx* c, const double* gammaFace, const double*
       info->converged = allConv ? 1 : 0;
       info->outer = nOuter;
       info->final_res_norm = std::sqrt(std::max(sc[4], 0.0));
-      // eps = max(atol, rtol |b|) is not |b|; recompute |b| on the host from the assembled rhs
-      std::vector<double> hb(c->C);
-      CK(cudaMemcpy(hb.data(), c->pb, sizeof(double) * c->C, cudaMemcpyDeviceToHost));
-      double bn = 0.0;
-      for (double x : hb) bn += x * x;
-      info->final_rel_res = bn > 0.0 ? info->final_res_norm / std::sqrt(bn) : 0.0;
+      info->final_rel_res = sc[6] > 0.0 ? info->final_res_norm / sc[6] : 0.0;
     }
     return allConv ? ANB_OK : ANB_NOT_CONVERGED;
   });
@@ -1813,11 +1816,7 @@ int anb_scalar_transport_solve(anb_ctx* c, const double* flux, const double* gam
       info->converged = allConv ? 1 : 0;
       info->outer = nOuter;
       info->final_res_norm = sc[5];
-      std::vector<double> hb(c->C);
-      CK(cudaMemcpy(hb.data(), c->rhs, sizeof(double) * c->C, cudaMemcpyDeviceToHost));
-      double bn = 0.0;
-      for (double x : hb) bn += x * x;
-      info->final_rel_res = bn > 0.0 ? sc[5] / std::sqrt(bn) : 0.0;
+      info->final_rel_res = sc[6] > 0.0 ? sc[5] / sc[6] : 0.0;
     }
     return allConv ? ANB_OK : ANB_NOT_CONVERGED;
   });

@@ -143,7 +143,9 @@ struct anb_ctx {
   // scalar-library solves (allocated on first use)
   DevArena scalarArena;
   double *sMinv = nullptr, *sBcVal = nullptr, *sGamma = nullptr, *sFlux = nullptr, *sSrc = nullptr,
-         *sSp = nullptr, *sPhi = nullptr, *sGrad = nullptr;
+         *sSp = nullptr, *sPhi = nullptr, *sGrad = nullptr, *sRaw = nullptr;
+  int* sOrig = nullptr;
+  uint8_t* sFlip = nullptr;
   uint8_t* sBcType = nullptr;
   // steady sensitivities (adjoint_api.cu, allocated on first use)
   anb::AdjointData* adj = nullptr;

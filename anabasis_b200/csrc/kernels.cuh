@@ -199,6 +199,12 @@ struct ScalarArgs {
 };
 void launch_scalar_grad(const LaunchCfg& lc, const DMesh& m, const ScalarArgs& a);
 void launch_scalar_assemble(const LaunchCfg& lc, const DMesh& m, const ScalarArgs& a);
+// Moment inverse of the scalar gradient for the boundary types of a.bcType.
+void launch_scalar_minv(const LaunchCfg& lc, const DMesh& m, const ScalarArgs& a, double* minv);
+// dst[f] = src[orig[f]] (sign changed where flip, if orient) for internal faces, src[f] beyond.
+void launch_permute_faces(const LaunchCfg& lc, int nI, int nF, const int* orig, const uint8_t* flip, bool orient,
+                          const double* src, double* dst);
+void launch_fill(const LaunchCfg& lc, int n, double v, double* dst);
 
 struct NonOrthArgs {
   const double* rau;
@@ -255,7 +261,7 @@ struct BicgArgsT {
   const T* b;
   T* x;
   T *r, *rh, *p, *v, *s, *t, *ph, *sh;
-  double* sc;         // per component 8 scalars: rho, rhoN, alpha, omega, eps, rn, tsum, ssum
+  double* sc;         // per component 8 scalars: rho, rhoN, alpha, omega, eps, rn, |b|, -
   int* fl;            // per component 4 ints: done, half, iters, converged; fl[12]: loop-graph trips
   double atol, rtol;
   int maxit;
@@ -307,7 +313,7 @@ struct PcgArgsT {
   T* r2;
   int mode;           // 0: PCG iteration; 1: plain preconditioner application z = M^-1 r (no update of
                       // x or r, no r.z reduction; fl[0] is the caller's done flag)
-  double* sc;         // rz, alpha, beta, eps, rr, pq
+  double* sc;         // rz, alpha, beta, eps, rr, pq, |b|
   int* fl;            // done, iters, converged, first, loop-graph trips (pcg_capture_loop)
   double atol, rtol;
   int maxit;

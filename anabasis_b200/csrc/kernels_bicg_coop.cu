@@ -43,7 +43,7 @@ __device__ __forceinline__ void add_release(unsigned* p) {
 
 // Recurrence scalars and flags of a component, kept by every block (one thread updates them).
 struct CoopState {
-  double eps, rn, rhoN, rho, al, om;
+  double eps, rn, bn, rhoN, rho, al, om;
   int done, half, its, conv;
 };
 
@@ -169,7 +169,8 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_bicg_coop(BicgArgs a, int m
     q2[1] += b * b;
   }
   if (!grid_sum<2>(bar, sh, epoch, nc, q2, [&](CoopState& c, const double* sum) {
-        c.eps = fmax(a.atol, a.rtol * sqrt(sum[1]));
+        c.bn = sqrt(sum[1]);
+        c.eps = fmax(a.atol, a.rtol * c.bn);
         c.rn = sqrt(sum[0]);
         c.rhoN = sum[0];
         c.rho = c.al = c.om = 1.0;
@@ -285,6 +286,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_bicg_coop(BicgArgs a, int m
     const CoopState& c = sh.st[threadIdx.x];
     a.sc[8 * threadIdx.x + 4] = c.eps;
     a.sc[8 * threadIdx.x + 5] = c.rn;
+    a.sc[8 * threadIdx.x + 6] = c.bn;
     int* f = a.fl + 4 * threadIdx.x;
     f[0] = 1;
     f[1] = c.half;

@@ -90,7 +90,7 @@ __device__ __forceinline__ void row3(const DSellT<T>& A, int r, const T* x, size
 }
 
 // ---------------------------------------------------------------- BiCGSTAB, nc components
-// scalars per component c: sc[8c + 0..7] = rho, rhoN, alpha, omega, eps, rn, -, -
+// scalars per component c: sc[8c + 0..7] = rho, rhoN, alpha, omega, eps, rn, |b|, -
 // flags per component c:   fl[4c + 0..3] = done, half, iters, converged
 // Component loops run over the constant bound 3 with `c < nc` as a guard: with a run-time bound
 // the per-component arrays (flags, scalars, partial sums) are indexed dynamically and live in
@@ -138,6 +138,7 @@ __global__ void __launch_bounds__(kBlock) k_bicg_init(BicgArgsT<T> a) {
       const double bn = sqrt(acc[2 * c + 1]);
       s[4] = fmax(a.atol, a.rtol * bn);
       s[5] = sqrt(acc[2 * c]);
+      s[6] = bn;
       s[0] = 1.0;
       s[1] = acc[2 * c];
       s[2] = 1.0;
@@ -375,6 +376,7 @@ __global__ void __launch_bounds__(kBlock) k_pcg_init(PcgArgsT<T> a) {
   if (grid_reduce<2>(acc, 0u, a.red, sm) && threadIdx.x == 0) {
     a.sc[3] = fmax(a.atol, a.rtol * sqrt(acc[1]));
     a.sc[4] = acc[0];
+    a.sc[6] = sqrt(acc[1]);
     a.sc[2] = 0.0;
     a.fl[0] = sqrt(acc[0]) <= a.sc[3] ? 1 : 0;
     a.fl[1] = 0;
