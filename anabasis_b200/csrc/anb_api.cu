@@ -7,6 +7,7 @@
 #include <memory>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "context.hpp"
@@ -468,7 +469,7 @@ bool build_sa(anb_ctx* c, AmgDevT<T>& A, DevArena& ar, T* val0, T* diag0, T* wdi
   auto reset = [&](bool ok) {
     if (ok) return true;
     CK(cudaStreamSynchronize(c->stream));
-    ar.release();
+    ar.recycle();
     A.nLevels = 0;
     A.sa = 0;
     return false;
@@ -496,12 +497,13 @@ bool build_sa(anb_ctx* c, AmgDevT<T>& A, DevArena& ar, T* val0, T* diag0, T* wdi
     for (int tries = 0;; ++tries, theta *= 0.5) {
       std::vector<int> agg = sa_aggregate(M, theta, nc);
       if (nc < 1 || nc > (int)(0.9 * M.n)) return reset(false);
+      if (tries < 3 && sa_next_entries(M, agg, nc) > 1.25 * M.col.size()) continue;
       S = sa_pattern(M, std::move(agg), nc, l > 0);
       f.capQ = f.capC = 1;
       for (int i = 0; i < M.n; ++i) f.capQ = std::max(f.capQ, S.qOff[i + 1] - S.qOff[i]);
       for (int I = 0; I < nc; ++I) f.capC = std::max(f.capC, S.cOff[I + 1] - S.cOff[I] + 1);
       const bool fits = sa_product_smem(8, 256, std::max(f.capQ, f.capC)) <= kSaSmemMax;
-      if (fits && (S.cCol.size() <= M.col.size() * 5 / 4 || tries == 3)) break;
+      if (fits) break;
       if (tries == 3) return reset(false);
     }
     AmgLevelDevT<T>& k = A.lv[l + 1];
@@ -517,7 +519,8 @@ bool build_sa(anb_ctx* c, AmgDevT<T>& A, DevArena& ar, T* val0, T* diag0, T* wdi
     f.ptOff = ar.upload(S.ptOff);
     f.ptCol = ar.upload(S.ptCol);
     f.ptSrc = ar.upload(S.ptSrc);
-    if (l == 0) {  // Q in SELL-32 (columns padded with 0, never read)
+    int* qColS = nullptr;
+    if (l == 0) {  // Q in SELL-32 (padding is never read)
       const int nSl = (M.n + kSlice - 1) / kSlice;
       std::vector<int> sl(nSl + 1, 0);
       for (int s = 0; s < nSl; ++s) {
@@ -525,14 +528,10 @@ bool build_sa(anb_ctx* c, AmgDevT<T>& A, DevArena& ar, T* val0, T* diag0, T* wdi
         for (int i = s * kSlice; i < std::min(M.n, (s + 1) * kSlice); ++i) w = std::max(w, S.qOff[i + 1] - S.qOff[i]);
         sl[s + 1] = sl[s] + w * kSlice;
       }
-      std::vector<int> cs(sl[nSl], 0);
-#pragma omp parallel for schedule(static)
-      for (int i = 0; i < M.n; ++i)
-        for (int e = S.qOff[i]; e < S.qOff[i + 1]; ++e)
-          cs[sl[i / kSlice] + (e - S.qOff[i]) * kSlice + i % kSlice] = S.qCol[e];
       f.qSlice = ar.upload(sl);
-      f.qColS = ar.upload(cs);
-      f.qVal = ar.alloc<T>(cs.size());
+      qColS = ar.alloc<int>(sl[nSl]);
+      f.qColS = qColS;
+      f.qVal = ar.alloc<T>(sl[nSl]);
       f.tOff = f.ptOff;
       f.tCol = f.ptCol;
       f.tSrc = f.ptSrc;
@@ -556,6 +555,9 @@ bool build_sa(anb_ctx* c, AmgDevT<T>& A, DevArena& ar, T* val0, T* diag0, T* wdi
     k.b = ar.alloc<T>(nc);
     k.x = ar.alloc<T>(nc);
     k.x2 = ar.alloc<T>(nc);
+    // the uploads' last DMA may still be under way, and the context's stream does not wait for them
+    CK(cudaStreamSynchronize(cudaStreamLegacy));
+    if (qColS) launch_sa_sell_cols(c->lc, M.n, f.qOff, f.qCol, f.qSlice, qColS);
     sa_refresh_level(c->lc, A, l);
     std::vector<T> v(S.cCol.size()), dg(nc);
     CK(cudaMemcpyAsync(v.data(), k.val, v.size() * sizeof(T), cudaMemcpyDeviceToHost, c->stream));
@@ -585,7 +587,14 @@ void build_amg(anb_ctx* c, AmgDevT<T>& A, std::vector<AmgLevelHost>& H, DevArena
   CK(cudaMemcpyAsync(hv.data(), val0, hv.size() * sizeof(T), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaMemcpyAsync(hd.data(), diag0, hd.size() * sizeof(T), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  std::vector<double> hvd(hv.begin(), hv.end()), hdd(hd.begin(), hd.end());
+  std::vector<double> hvd, hdd;
+  if constexpr (std::is_same_v<T, double>) {
+    hvd.swap(hv);
+    hdd.swap(hd);
+  } else {
+    hvd.assign(hv.begin(), hv.end());
+    hdd.assign(hd.begin(), hd.end());
+  }
   const char* noGraph = std::getenv("ANB_NO_GRAPH");
   if (ga && build_sa(c, A, ar, val0, diag0, wdinv0, hvd, hdd)) {
     H.clear();
@@ -656,6 +665,7 @@ void build_amg(anb_ctx* c, AmgDevT<T>& A, std::vector<AmgLevelHost>& H, DevArena
   A.nDense = nd;
   A.dense = ar.alloc<double>((size_t)nd * nd);
   if (ga) c->amgBuilt = true;
+  CK(cudaStreamSynchronize(cudaStreamLegacy));  // the uploads, before the context's stream reads them
   const char* tailEnv = std::getenv("ANB_AMG_TAIL_ROWS");
   amg_configure_tail(A, tailEnv ? std::atoi(tailEnv) : kAmgTailRows, c->stream);
   const char* fdEnv = std::getenv("ANB_AMG_FUSED_DOWN_ROWS");
@@ -1084,7 +1094,7 @@ void release_amg(anb_ctx* c) {
   amg_release_graphs(c->amg32);
   c->amg32.nLevels = c->amg32.sa = 0;
   c->amg32.dense = nullptr;
-  c->amgArena.release();
+  c->amgArena.recycle();
   c->amgHost.clear();
   c->amgBuilt = false;
 }

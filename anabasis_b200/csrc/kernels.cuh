@@ -417,6 +417,8 @@ inline size_t sa_product_smem(int G, int TS, int cap) {
   return (size_t)(kBlock / TS) * cap * ((size_t)(TS / G) * sizeof(double) + sizeof(int));
 }
 inline bool sa_small_team(int rows, int cap) { return rows >= 16384 && sa_product_smem(4, 32, cap) <= kSaSmemMax; }
+// Columns of a CSR pattern in SELL-32 order (slice offsets given).
+void launch_sa_sell_cols(const LaunchCfg& lc, int n, const int* off, const int* col, const int* slice, int* out);
 template <class T>
 void sa_configure_tail(AmgDevT<T>& amg, int tailRows, cudaStream_t s);
 template <class T>

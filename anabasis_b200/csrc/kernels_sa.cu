@@ -425,6 +425,14 @@ __global__ void __launch_bounds__(kBlock) k_sa_product(AmgLevelDevT<T> f, AmgLev
   }
 }
 
+__global__ void __launch_bounds__(kBlock) k_sa_sell_cols(int n, const int* off, const int* col, const int* slice,
+                                                         int* out) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int k0 = off[i], k1 = off[i + 1], b = slice[i >> 5] + (i & 31);
+    for (int k = k0; k < k1; ++k) out[b + ((k - k0) << 5)] = col[k];
+  }
+}
+
 template <class T>
 __global__ void __launch_bounds__(kBlock) k_sa_gather(int n, const int* src, const T* v, T* out) {
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) out[e] = v[src[e]];
@@ -492,6 +500,11 @@ void with_lanes(int g, F&& fn) {
 }
 
 }  // namespace
+
+void launch_sa_sell_cols(const LaunchCfg& lc, int n, const int* off, const int* col, const int* slice, int* out) {
+  g_launches += 1;
+  k_sa_sell_cols<<<grid_for(n, 1 << 30), kBlock, 0, lc.stream>>>(n, off, col, slice, out);
+}
 
 template <int G, int TS, bool kAP, class T>
 static void launch_product(const LaunchCfg& lc, const AmgLevelDevT<T>& f, const AmgLevelDevT<T>& c, double omega,

@@ -42,21 +42,42 @@ void build_rows(int n, int marks, std::vector<int>& off, std::vector<int>& col, 
   }
 }
 
-// Rows of the transpose (nc rows), each in ascending order of the original row.
+// Rows of the transpose (nc rows), each in ascending order of the original row.  Threads count and
+// then place contiguous row ranges, one after the other within every row of the transpose.
 void transpose(int n, int nc, const std::vector<int>& off, const std::vector<int>& col, std::vector<int>& tOff,
                std::vector<int>& tCol, std::vector<int>& tSrc) {
   tOff.assign((size_t)nc + 1, 0);
-  for (int c : col) tOff[c + 1]++;
-  for (int I = 0; I < nc; ++I) tOff[I + 1] += tOff[I];
-  std::vector<int> fill(tOff.begin(), tOff.end() - 1);
   tCol.resize(col.size());
   tSrc.resize(col.size());
-  for (int i = 0; i < n; ++i)
-    for (int k = off[i]; k < off[i + 1]; ++k) {
-      const int s = fill[col[k]]++;
-      tCol[s] = i;
-      tSrc[s] = k;
+  const int most = std::max(1, std::min(omp_get_max_threads(), n / 4096));
+  std::vector<std::vector<int>> cnt(most);
+#pragma omp parallel num_threads(most)
+  {
+    const int t = omp_get_thread_num(), T = omp_get_num_threads();
+    const int lo = (int)((long long)n * t / T), hi = (int)((long long)n * (t + 1) / T);
+    std::vector<int>& c = cnt[t];
+    c.assign(nc, 0);
+    for (int k = off[lo]; k < off[hi]; ++k) c[col[k]]++;
+#pragma omp barrier
+#pragma omp for schedule(static)
+    for (int I = 0; I < nc; ++I) {
+      int s = 0;
+      for (int u = 0; u < T; ++u) {
+        const int here = cnt[u][I];
+        cnt[u][I] = s;  // entries of the threads before
+        s += here;
+      }
+      tOff[I + 1] = s;
     }
+#pragma omp single
+    for (int I = 0; I < nc; ++I) tOff[I + 1] += tOff[I];
+    for (int i = lo; i < hi; ++i)
+      for (int k = off[i]; k < off[i + 1]; ++k) {
+        const int s = tOff[col[k]] + c[col[k]]++;
+        tCol[s] = i;
+        tSrc[s] = k;
+      }
+  }
 }
 
 }  // namespace
@@ -110,6 +131,51 @@ std::vector<int> sa_aggregate(const SaMatrix& A, double theta, int& nc) {
     agg[i] = ren[agg[i]];
   }
   return agg;
+}
+
+double sa_next_entries(const SaMatrix& A, const std::vector<int>& agg, int nc) {
+  const int n = A.n;
+  constexpr int kStep = 16;
+  std::vector<int> mOff((size_t)nc + 1, 0), mem(n);
+  for (int i = 0; i < n; ++i) mOff[agg[i] + 1]++;
+  for (int I = 0; I < nc; ++I) mOff[I + 1] += mOff[I];
+  {
+    std::vector<int> fill(mOff.begin(), mOff.end() - 1);
+    for (int i = 0; i < n; ++i) mem[fill[agg[i]]++] = i;
+  }
+  // row I of P^T A P reaches the aggregates of every row within three steps of I's rows
+  long long sum = 0;
+  const int rows = (nc + kStep - 1) / kStep;
+#pragma omp parallel reduction(+ : sum)
+  {
+    std::vector<char> seen(n, 0);
+    std::vector<int> met(nc, -1), q;
+#pragma omp for schedule(static)
+    for (int u = 0; u < rows; ++u) {
+      const int I = u * kStep;
+      q.assign(mem.begin() + mOff[I], mem.begin() + mOff[I + 1]);
+      for (int i : q) seen[i] = 1;
+      size_t from = 0;
+      for (int d = 0; d < 3; ++d) {
+        const size_t to = q.size();
+        for (; from < to; ++from)
+          for (int k = A.off[q[from]]; k < A.off[q[from] + 1]; ++k)
+            if (!seen[A.col[k]]) {
+              seen[A.col[k]] = 1;
+              q.push_back(A.col[k]);
+            }
+      }
+      for (int i : q) {
+        seen[i] = 0;
+        if (met[agg[i]] != I) {
+          met[agg[i]] = I;
+          ++sum;
+        }
+      }
+      --sum;  // the diagonal
+    }
+  }
+  return (double)sum / rows * nc;
 }
 
 SaPattern sa_pattern(const SaMatrix& A, std::vector<int> aggIn, int nc, bool wantQT) {

@@ -45,6 +45,8 @@ inline double sa_theta(int level, int n, int maxRowLen) {
 
 // Aggregate of every row; nc receives the count.  Aggregates are numbered by their first row.
 std::vector<int> sa_aggregate(const SaMatrix& A, double theta, int& nc);
+// Estimate of the next matrix's off-diagonal entries for these aggregates, from every 16th of its rows.
+double sa_next_entries(const SaMatrix& A, const std::vector<int>& agg, int nc);
 // All patterns of one level step for the given aggregates.
 SaPattern sa_pattern(const SaMatrix& A, std::vector<int> agg, int nc, bool wantQT);
 // The level-0 matrix as CSR; vals in the layout's SELL-32 storage.
