@@ -42,11 +42,16 @@ struct AdjointData {
   double rtol = 1e-10;  // relative tolerance of the tangent-linear and adjoint systems
   double momRtol = 1e-2, pRtol = 1e-2, schur = 1.0;
   int momMaxit = 200, momRelaxed = 1;
-  long long momIts = 0, pIts = 0;  // inner iterations since the last reset
+  long long momIts = 0, pIts = 0;  // inner iterations since the last reset, host-driven solves
+  int* cnt = nullptr;              // and those counted on the device (adj_count_prec)
+  double* hCoef = nullptr;         // pinned: Hessenberg column and counters of an FGMRES iteration
+  cudaGraphExec_t pLoop = nullptr; // the pressure solve's iterations (p_solve) as one launch
 };
 
 void adjoint_release(anb_ctx* c) {
   if (!c->adj) return;
+  if (c->adj->pLoop) cudaGraphExecDestroy(c->adj->pLoop);
+  if (c->adj->hCoef) cudaFreeHost(c->adj->hCoef);
   c->adj->ar.release();
   delete c->adj;
   c->adj = nullptr;
@@ -92,7 +97,10 @@ AdjointData& adj(anb_ctx* c) {
   d->muBar = A.alloc<double>(2);
   d->objVal = A.alloc<double>(2);
   d->partials = A.alloc<double>((size_t)c->lc.rowBlocks * (d->mBasis + 2));
-  d->coef = A.alloc<double>(d->mBasis + 2);
+  // h of the two Gram-Schmidt passes, the squared norm after them, and the work counters
+  d->coef = A.alloc<double>(2 * (size_t)(d->mBasis + 2) + 4);
+  d->cnt = reinterpret_cast<int*>(d->coef + 2 * (d->mBasis + 2) + 1);
+  CK(cudaMallocHost(&d->hCoef, sizeof(double) * (2 * (size_t)(d->mBasis + 2) + 4)));
   d->gX = A.alloc<double>(d->N);
   d->R = A.alloc<double>(d->N);
   d->t1 = A.alloc<double>(d->N);
@@ -176,6 +184,13 @@ void vjp(anb_ctx* c, AdjointData& d, const double* w, double* out) {
 }
 
 // ---- preconditioner ---------------------------------------------------------------------------
+PcgArgs p_args(anb_ctx* c, const AdjointData& d, const double* b) {
+  PcgArgs a = pcg_args(c, b, d.pRtol);
+  a.atol = 0.0;
+  a.maxit = 500;
+  return a;
+}
+
 // Momentum matrix at the converged state (relaxed as in the SIMPLE iteration, see AdjointData),
 // its transpose, the pressure matrix from the same rAU the SIMPLE iteration uses, and its AMG
 // hierarchy.
@@ -210,8 +225,12 @@ void prec_setup(anb_ctx* c, AdjointData& d) {
   pa.wdinv = c->pwdinv;
   pa.omega = c->amg.omega;
   launch_pressure_rc(c->lc, c->dm, pa);
+  if (d.pLoop) cudaGraphExecDestroy(d.pLoop);
+  d.pLoop = nullptr;
   release_amg(c);
   ensure_amg(c);
+  if (c->prm.p_use_amg && c->amgBuilt && c->amg.nLevels >= 2 && c->amg.loop)
+    pcg_capture_loop(c->lc, p_args(c, d, c->pb), c->amg, &d.pLoop);  // without it the host loop runs
   d.precReady = true;
 }
 
@@ -232,10 +251,9 @@ void mom_solve(anb_ctx* c, AdjointData& d, bool trans, const double* b, double* 
   a.maxit = d.momMaxit;
   a.red = c->red;
   CK(cudaMemsetAsync(x, 0, sizeof(double) * 3 * c->C, c->stream));
-  if (bicg_coop_solve(c->lc, a, 7, c->nSM, c->coopPart)) {
-    poll(c, a.fl, 14);
-    check_coop(c->hFlags);
-    d.momIts += std::max(c->hFlags[2], std::max(c->hFlags[6], c->hFlags[10]));
+  const int fam = c->prof.family;  // a timed kernel family runs from the host loops
+  if (fam != kKfBicgSpmv && fam != kKfBicgVector && bicg_coop_solve(c->lc, a, 7, c->nSM, c->coopPart)) {
+    adj_count_prec(c->lc, a.fl, nullptr, d.cnt);  // read with the iteration's Hessenberg column
     return;
   }
   bicg_init(c->lc, a);
@@ -251,13 +269,17 @@ void mom_solve(anb_ctx* c, AdjointData& d, bool trans, const double* b, double* 
 
 // x (C) = A_p^{-1} b, from x = 0 (the caller scales b)
 void p_solve(anb_ctx* c, AdjointData& d, const double* b, double* x) {
-  PcgArgs a = pcg_args(c, b, d.pRtol);
-  a.atol = 0.0;
-  a.maxit = 500;
+  const PcgArgs a = p_args(c, d, b);
   const AmgDev* amg = (c->prm.p_use_amg && c->amgBuilt && c->amg.nLevels >= 2) ? &c->amg : nullptr;
   CK(cudaMemsetAsync(a.x, 0, sizeof(double) * c->C, c->stream));
   pcg_init(c->lc, a);
   pcg_precondition(c->lc, a, amg);
+  const int fam = c->prof.family;
+  if (d.pLoop && !(fam >= kKfPcgSpmv && fam <= kKfPcgUpdate) && cudaGraphLaunch(d.pLoop, c->stream) == cudaSuccess) {
+    CK(cudaMemcpyAsync(x, a.x, sizeof(double) * c->C, cudaMemcpyDeviceToDevice, c->stream));
+    adj_count_prec(c->lc, nullptr, a.fl, d.cnt);
+    return;
+  }
   int it = 0;
   while (true) {
     for (int k = 0; k < 8; ++k) pcg_iteration(c->lc, a, it++, amg);
@@ -268,14 +290,12 @@ void p_solve(anb_ctx* c, AdjointData& d, const double* b, double* x) {
   d.pIts += c->hFlags[1];
 }
 
-void scale(anb_ctx* c, AdjointData& d, size_t n, const double* src, double s, double* dst) {
-  CK(cudaMemcpyAsync(d.coef, &s, sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  vec_lincomb(c->lc, n, 1, src, n, d.coef, 0.0, dst);
+void scale(anb_ctx* c, AdjointData&, size_t n, const double* src, double s, double* dst) {
+  vec_axpby(c->lc, n, s, src, 0.0, dst);
 }
-// dst = a * x + b * y  (n)
-void axpby(anb_ctx* c, AdjointData& d, size_t n, double a, const double* x, double b, double* y) {
-  CK(cudaMemcpyAsync(d.coef, &a, sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  vec_lincomb(c->lc, n, 1, x, n, d.coef, b, y);
+// y = a x + b y (n)
+void axpby(anb_ctx* c, AdjointData&, size_t n, double a, const double* x, double b, double* y) {
+  vec_axpby(c->lc, n, a, x, b, y);
 }
 
 // z = P^{-1} s (forward) or P^{-T} s (transposed); s, z: 4C.  Uses t1..t3 as work.
@@ -336,7 +356,7 @@ KrylovResult fgmres(anb_ctx* c, AdjointData& d, bool trans, const double* b, dou
     return kr;
   }
   const double target = rtol * kr.bnorm;
-  std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), gvec(m + 1), y(m), hcol(m + 2), h2(m + 2);
+  std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), gvec(m + 1), y(m), hcol(m + 2);
   bool first = true;
   while (kr.its < maxIt) {
     // r = b - K x (the first cycle starts from x = 0)
@@ -368,21 +388,21 @@ KrylovResult fgmres(anb_ctx* c, AdjointData& d, bool trans, const double* b, dou
       if (trans) vjp(c, d, zj, w);
       else jvp(c, d, zj, d.dgZero, 0.0, w);
       ++kr.its;
-      // classical Gram-Schmidt, twice
+      // classical Gram-Schmidt, twice, and the norm: the coefficients stay on the device, one read-back
+      const int ldc = m + 2;
       for (int pass = 0; pass < 2; ++pass) {
-        vec_mdot(c->lc, N, j + 1, d.V, N, w, d.partials, d.coef);
-        CK(cudaMemcpyAsync(h2.data(), d.coef, sizeof(double) * (j + 1), cudaMemcpyDeviceToHost, c->stream));
-        CK(cudaStreamSynchronize(c->stream));
-        for (int i = 0; i <= j; ++i) {
-          hcol[i] = (pass ? hcol[i] : 0.0) + h2[i];
-          h2[i] = -h2[i];
-        }
-        CK(cudaMemcpyAsync(d.coef, h2.data(), sizeof(double) * (j + 1), cudaMemcpyHostToDevice, c->stream));
-        vec_lincomb(c->lc, N, j + 1, d.V, N, d.coef, 1.0, w);
+        vec_mdot(c->lc, N, j + 1, d.V, N, w, d.partials, d.coef + pass * ldc);
+        vec_lincomb(c->lc, N, j + 1, d.V, N, d.coef + pass * ldc, -1.0, 1.0, w);
       }
-      const double hn = norm(c, d, N, w);
+      vec_mdot(c->lc, N, 1, w, N, w, d.partials, d.coef + 2 * ldc);
+      vec_unit(c->lc, N, d.coef + 2 * ldc, w);
+      CK(cudaMemcpyAsync(d.hCoef, d.coef, sizeof(double) * (2 * ldc + 4), cudaMemcpyDeviceToHost, c->stream));
+      CK(cudaStreamSynchronize(c->stream));
+      if (reinterpret_cast<const int*>(d.hCoef + 2 * ldc + 1)[2])
+        throw AnbError(ANB_ERR_CUDA, "a grid barrier of the BiCGSTAB kernel timed out");
+      for (int i = 0; i <= j; ++i) hcol[i] = d.hCoef[i] + d.hCoef[ldc + i];
+      const double hn = std::sqrt(std::max(d.hCoef[2 * ldc], 0.0));
       hcol[j + 1] = hn;
-      if (hn > 0.0) scale(c, d, N, w, 1.0 / hn, w);
       // Givens rotations
       for (int i = 0; i < j; ++i) {
         const double t = cs[i] * hcol[i] + sn[i] * hcol[i + 1];
@@ -410,7 +430,7 @@ KrylovResult fgmres(anb_ctx* c, AdjointData& d, bool trans, const double* b, dou
       y[i] = H[(size_t)i * m + i] != 0.0 ? s / H[(size_t)i * m + i] : 0.0;
     }
     CK(cudaMemcpyAsync(d.coef, y.data(), sizeof(double) * j, cudaMemcpyHostToDevice, c->stream));
-    vec_lincomb(c->lc, N, j, d.Z, N, d.coef, 1.0, x);
+    vec_lincomb(c->lc, N, j, d.Z, N, d.coef, 1.0, 1.0, x);
     if (kr.res <= target) {
       // confirm with the true residual
       if (trans) vjp(c, d, x, d.t3);
@@ -440,12 +460,19 @@ ObjArgs obj_args(anb_ctx* c, AdjointData& d, int patch, int sign, const double d
   return o;
 }
 
-void fill_info(anb_adjoint_info* info, const KrylovResult& kr, double secs, const AdjointData* d = nullptr) {
+// Starts the count of the preconditioner's iterations.
+void reset_work(anb_ctx* c, AdjointData& d) {
+  d.momIts = d.pIts = 0;
+  CK(cudaMemsetAsync(d.cnt, 0, 4 * sizeof(int), c->stream));
+}
+
+void fill_info(anb_ctx* c, anb_adjoint_info* info, const KrylovResult& kr, double secs, const AdjointData& d) {
   if (!info) return;
-  if (d) {
-    info->prec_mom_its = (int)d->momIts;
-    info->prec_p_its = (int)d->pIts;
-  }
+  int n[3] = {0, 0, 0};
+  CK(cudaMemcpyAsync(n, d.cnt, sizeof(n), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  info->prec_mom_its = (int)d.momIts + n[0];
+  info->prec_p_its = (int)d.pIts + n[1];
   info->iterations = kr.its;
   info->converged = kr.conv ? 1 : 0;
   info->res_norm = kr.res;
@@ -577,7 +604,7 @@ int anb_newton_solve(anb_ctx* c, int maxNewton, double tol, int linMaxIt, int* s
     require(c);
     const auto t0 = std::chrono::steady_clock::now();
     AdjointData& d = adj(c);
-    d.momIts = d.pIts = 0;
+    reset_work(c, d);
     KrylovResult kr{};
     int k = 0, total = 0;
     double rn = 0.0;
@@ -598,7 +625,7 @@ int anb_newton_solve(anb_ctx* c, int maxNewton, double tol, int linMaxIt, int* s
     if (resNorm) *resNorm = rn;
     kr.its = total;
     kr.res = rn;
-    fill_info(info, kr, seconds_since(t0), &d);
+    fill_info(c, info, kr, seconds_since(t0), d);
     if (info) info->converged = rn <= tol ? 1 : 0;
     return rn <= tol ? ANB_OK : ANB_NOT_CONVERGED;
   });
@@ -611,7 +638,7 @@ int anb_tangent_linear(anb_ctx* c, int patch, int sign, const double dir[3], con
     require(c);
     const auto t0 = std::chrono::steady_clock::now();
     AdjointData& d = adj(c);
-    d.momIts = d.pIts = 0;
+    reset_work(c, d);
     base(c, d);
     prec_setup(c, d);
     upload_bc3(c, dbc, d.dgDir);
@@ -626,7 +653,7 @@ int anb_tangent_linear(anb_ctx* c, int patch, int sign, const double dir[3], con
     CK(cudaMemcpyAsync(v, d.objVal, sizeof(v), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     *dJ = jx + v[1] * dmu;
-    fill_info(info, kr, seconds_since(t0), &d);
+    fill_info(c, info, kr, seconds_since(t0), d);
     return kr.conv ? ANB_OK : ANB_NOT_CONVERGED;
   });
 }
@@ -638,7 +665,7 @@ int anb_adjoint_force_grad(anb_ctx* c, int patch, int sign, const double dir[3],
     require(c);
     const auto t0 = std::chrono::steady_clock::now();
     AdjointData& d = adj(c);
-    d.momIts = d.pIts = 0;
+    reset_work(c, d);
     base(c, d);
     prec_setup(c, d);
     adj_objective(c->lc, c->dm, adj_args(c, d), obj_args(c, d, patch, sign, dir), d.gX);
@@ -655,7 +682,7 @@ int anb_adjoint_force_grad(anb_ctx* c, int patch, int sign, const double dir[3],
       const size_t n = (size_t)3 * (c->nI + c->nB);
       for (size_t i = 0; i < n; ++i) dJ_dbc[i] = -dJ_dbc[i];
     }
-    fill_info(info, kr, seconds_since(t0), &d);
+    fill_info(c, info, kr, seconds_since(t0), d);
     return kr.conv ? ANB_OK : ANB_NOT_CONVERGED;
   });
 }

@@ -442,6 +442,9 @@ cudaError_t amg_capture_graph(const LaunchCfg& lc, const PcgArgsT<T>& a, AmgDevT
 // iterations were enqueued on the device).
 template <class T>
 bool pcg_loop_launch(const LaunchCfg& lc, const PcgArgsT<T>& a, const AmgDevT<T>& amg);
+// The same loop captured for other arguments a (another iteration cap) into *out.
+template <class T>
+cudaError_t pcg_capture_loop(const LaunchCfg& lc, const PcgArgsT<T>& a, const AmgDevT<T>& amg, cudaGraphExec_t* out);
 // Destroys the captured V-cycles and the loop graph (the stream must be idle).
 template <class T>
 void amg_release_graphs(AmgDevT<T>& amg);
@@ -520,8 +523,14 @@ void adj_permute(const LaunchCfg& lc, int n, const int* idx, const double* src, 
 // out[j] = V_j . x for j < k (V: k vectors of length n, stride ld); partials: rowBlocks * k
 void vec_mdot(const LaunchCfg& lc, size_t n, int k, const double* V, size_t ld, const double* x, double* partials,
               double* out);
-// x = beta x + sum_j coef[j] V_j (coef on the device)
-void vec_lincomb(const LaunchCfg& lc, size_t n, int k, const double* V, size_t ld, const double* coef, double beta,
-                 double* x);
+// x = beta x + sgn sum_j coef[j] V_j (coef on the device)
+void vec_lincomb(const LaunchCfg& lc, size_t n, int k, const double* V, size_t ld, const double* coef, double sgn,
+                 double beta, double* x);
+// y = a x + b y; x /= sqrt(*sq) (sq on the device; left alone when that is not positive)
+void vec_axpby(const LaunchCfg& lc, size_t n, double a, const double* x, double b, double* y);
+void vec_unit(const LaunchCfg& lc, size_t n, const double* sq, double* x);
+// Adds the iterations in the flags of a momentum and / or a pressure solve to cnt[0], cnt[1]; cnt[2]
+// takes the momentum kernel's time-out flag.
+void adj_count_prec(const LaunchCfg& lc, const int* mom, const int* pres, int* cnt);
 
 }  // namespace anb

@@ -642,35 +642,65 @@ __global__ void __launch_bounds__(kBlock) k_permute(int n, const int* idx, const
 
 // ---- vector kernels for the Krylov solver (deterministic: fixed partition, fixed order) ----
 // partials[j * gridDim.x + block] = sum over the block's rows of V_j . x, j < k
+constexpr int kMdot = 4;  // vectors of a k_mdot_partial block (blockIdx.y counts the groups of four)
 __global__ void __launch_bounds__(kBlock) k_mdot_partial(size_t n, int k, const double* V, size_t ld, const double* x,
                                                          double* partials) {
-  __shared__ double sm[32];
-  for (int j = 0; j < k; ++j) {
-    double v[1] = {0.0};
-    const double* Vj = V + (size_t)j * ld;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-      v[0] += Vj[i] * x[i];
-    block_reduce<1>(v, 0u, sm);
-    if (threadIdx.x == 0) partials[(size_t)j * gridDim.x + blockIdx.x] = v[0];
+  __shared__ double sm[kMdot * 32];
+  const int j0 = blockIdx.y * kMdot;
+  const double* Vj[kMdot];
+#pragma unroll
+  for (int q = 0; q < kMdot; ++q) Vj[q] = V + (size_t)min(j0 + q, k - 1) * ld;
+  double v[kMdot] = {0.0, 0.0, 0.0, 0.0};
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const double xi = x[i];
+#pragma unroll
+    for (int q = 0; q < kMdot; ++q) v[q] += Vj[q][i] * xi;
   }
+  block_reduce<kMdot>(v, 0u, sm);
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int q = 0; q < kMdot; ++q)
+      if (j0 + q < k) partials[(size_t)(j0 + q) * gridDim.x + blockIdx.x] = v[q];
 }
-__global__ void k_mdot_final(int k, int nb, const double* partials, double* out) {
+// out[j] for j = blockIdx.x
+__global__ void __launch_bounds__(kBlock) k_mdot_final(int nb, const double* partials, double* out) {
   __shared__ double sm[32];
-  for (int j = 0; j < k; ++j) {
-    double v[1] = {0.0};
-    for (int b = threadIdx.x; b < nb; b += blockDim.x) v[0] += partials[(size_t)j * nb + b];
-    block_reduce<1>(v, 0u, sm);
-    if (threadIdx.x == 0) out[j] = v[0];
-  }
+  const int j = blockIdx.x;
+  double v[1] = {0.0};
+  for (int b = threadIdx.x; b < nb; b += blockDim.x) v[0] += partials[(size_t)j * nb + b];
+  block_reduce<1>(v, 0u, sm);
+  if (threadIdx.x == 0) out[j] = v[0];
 }
-// x = beta x + sum_j coef[j] V_j
+// x = beta x + sgn sum_j coef[j] V_j
 __global__ void __launch_bounds__(kBlock) k_lincomb(size_t n, int k, const double* V, size_t ld, const double* coef,
-                                                    double beta, double* x) {
+                                                    double sgn, double beta, double* x) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     double s = beta == 0.0 ? 0.0 : beta * x[i];
-    for (int j = 0; j < k; ++j) s += coef[j] * V[(size_t)j * ld + i];
+#pragma unroll 8
+    for (int j = 0; j < k; ++j) s += (sgn * coef[j]) * V[(size_t)j * ld + i];
     x[i] = s;
   }
+}
+// y = a x + b y (b = 0: y is not read)
+__global__ void __launch_bounds__(kBlock) k_axpby(size_t n, double a, const double* x, double b, double* y) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    y[i] = b == 0.0 ? a * x[i] : a * x[i] + b * y[i];
+}
+// x /= sqrt(*sq) (unless that is not positive)
+__global__ void __launch_bounds__(kBlock) k_unit(size_t n, const double* sq, double* x) {
+  const double h = sqrt(fmax(*sq, 0.0));
+  if (!(h > 0.0)) return;
+  const double s = 1.0 / h;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) x[i] *= s;
+}
+// Preconditioner work of one application: cnt[0] += momentum iterations (the most of the components),
+// cnt[1] += pressure iterations, cnt[2] |= a barrier of the momentum kernel timed out.
+__global__ void k_count_prec(const int* mom, const int* pres, int* cnt) {
+  if (mom) {
+    cnt[0] += max(mom[2], max(mom[6], mom[10]));
+    cnt[2] |= mom[13];
+  }
+  if (pres) cnt[1] += pres[1];
 }
 
 }  // namespace
@@ -725,13 +755,25 @@ void vec_mdot(const LaunchCfg& lc, size_t n, int k, const double* V, size_t ld, 
               double* out) {
   g_launches += 2;
   const int nb = blocks(lc);
-  k_mdot_partial<<<nb, kBlock, 0, lc.stream>>>(n, k, V, ld, x, partials);
-  k_mdot_final<<<1, 1024, 0, lc.stream>>>(k, nb, partials, out);
+  k_mdot_partial<<<dim3(nb, (k + kMdot - 1) / kMdot), kBlock, 0, lc.stream>>>(n, k, V, ld, x, partials);
+  k_mdot_final<<<k, kBlock, 0, lc.stream>>>(nb, partials, out);
 }
-void vec_lincomb(const LaunchCfg& lc, size_t n, int k, const double* V, size_t ld, const double* coef, double beta,
-                 double* x) {
+void vec_lincomb(const LaunchCfg& lc, size_t n, int k, const double* V, size_t ld, const double* coef, double sgn,
+                 double beta, double* x) {
   g_launches += 1;
-  k_lincomb<<<blocks(lc), kBlock, 0, lc.stream>>>(n, k, V, ld, coef, beta, x);
+  k_lincomb<<<blocks(lc), kBlock, 0, lc.stream>>>(n, k, V, ld, coef, sgn, beta, x);
+}
+void vec_axpby(const LaunchCfg& lc, size_t n, double a, const double* x, double b, double* y) {
+  g_launches += 1;
+  k_axpby<<<blocks(lc), kBlock, 0, lc.stream>>>(n, a, x, b, y);
+}
+void vec_unit(const LaunchCfg& lc, size_t n, const double* sq, double* x) {
+  g_launches += 1;
+  k_unit<<<blocks(lc), kBlock, 0, lc.stream>>>(n, sq, x);
+}
+void adj_count_prec(const LaunchCfg& lc, const int* mom, const int* pres, int* cnt) {
+  g_launches += 1;
+  k_count_prec<<<1, 1, 0, lc.stream>>>(mom, pres, cnt);
 }
 
 }  // namespace anb

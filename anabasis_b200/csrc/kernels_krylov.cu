@@ -1205,9 +1205,6 @@ void pcg_precondition(const LaunchCfg& lc, const PcgArgsT<T>& a, const AmgDevT<T
 // read is fixed for the life of the hierarchy (values change on refresh, addresses do not; the
 // callers keep x, r, r2, p0, p1, q and z at fixed addresses), so the graphs are captured once and
 // replayed for every preconditioner application.
-template <class T>
-static cudaError_t pcg_capture_loop(const LaunchCfg& lc, const PcgArgsT<T>& a, AmgDevT<T>& amg);
-
 // ANB_NO_LOOP_GRAPH=1 keeps the solver loops on the host (for measurements)
 static bool loop_graphs_off() {
   const char* s = std::getenv("ANB_NO_LOOP_GRAPH");
@@ -1233,7 +1230,11 @@ cudaError_t amg_capture_graph(const LaunchCfg& lc, const PcgArgsT<T>& a, AmgDevT
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return e;
   }
-  if (a.mode == 0 && !loop_graphs_off()) pcg_capture_loop(lc, a, amg);  // else the host loop runs
+  if (a.mode == 0 && !loop_graphs_off()) {  // else the host loop runs
+    if (amg.loop) cudaGraphExecDestroy(amg.loop);
+    amg.loop = nullptr;
+    if (pcg_capture_loop(lc, a, amg, &amg.loop) == cudaSuccess) amg.loopArgs = a;
+  }
   return cudaSuccess;
 }
 
@@ -1302,13 +1303,11 @@ static cudaError_t capture_while(cudaStream_t s, Body&& body, Cond&& cond, cudaG
 // convergence return at once, as in the host loop.  The kernels are those of pcg_iteration with
 // the same arguments, so the iterates are the same bit for bit.
 template <class T>
-static cudaError_t pcg_capture_loop(const LaunchCfg& lc, const PcgArgsT<T>& a, AmgDevT<T>& amg) {
-  if (amg.loop) cudaGraphExecDestroy(amg.loop);
-  amg.loop = nullptr;
+cudaError_t pcg_capture_loop(const LaunchCfg& lc, const PcgArgsT<T>& a, const AmgDevT<T>& amg, cudaGraphExec_t* out) {
   LaunchCfg quiet = lc;
   quiet.prof = nullptr;
   const int maxTrips = a.maxit / 2 + 3;
-  const cudaError_t e = capture_while(
+  return capture_while(
       lc.stream,
       [&] {
         for (int it = 0; it < 2; ++it) {
@@ -1316,10 +1315,7 @@ static cudaError_t pcg_capture_loop(const LaunchCfg& lc, const PcgArgsT<T>& a, A
           vcycle(quiet, a, &amg, (it + 1) & 1);
         }
       },
-      [&](cudaGraphConditionalHandle h) { k_pcg_loop_cond<<<1, 1, 0, lc.stream>>>(h, a.fl, maxTrips); },
-      &amg.loop);
-  if (e == cudaSuccess) amg.loopArgs = a;
-  return e;
+      [&](cudaGraphConditionalHandle h) { k_pcg_loop_cond<<<1, 1, 0, lc.stream>>>(h, a.fl, maxTrips); }, out);
 }
 
 template <class T>
@@ -1484,6 +1480,8 @@ void launch_apply_correction(const LaunchCfg& lc, int n, int nc, double* x, floa
   template void amg_dense_factor<T>(const LaunchCfg&, const AmgLevelDevT<T>&, double*);        \
   template cudaError_t amg_capture_graph<T>(const LaunchCfg&, const PcgArgsT<T>&, AmgDevT<T>&);           \
   template bool pcg_loop_launch<T>(const LaunchCfg&, const PcgArgsT<T>&, const AmgDevT<T>&);  \
+  template cudaError_t pcg_capture_loop<T>(const LaunchCfg&, const PcgArgsT<T>&, const AmgDevT<T>&,           \
+                                           cudaGraphExec_t*);                                                   \
   template void amg_release_graphs<T>(AmgDevT<T>&);                                           \
   template bool bicg_loop_launch<T>(const LaunchCfg&, const BicgArgsT<T>&, BicgLoopT<T>&);     \
   template void bicg_loop_release<T>(BicgLoopT<T>&);                                          \
