@@ -537,15 +537,30 @@ bool build_sa(anb_ctx* c, AmgDevT<T>& A, DevArena& ar, T* val0, T* diag0, T* wdi
       f.tSrc = f.ptSrc;
       f.nT = (int)S.ptCol.size();
     } else {
-      f.qVal = ar.alloc<T>(S.qCol.size());
+      // merged rows [-w A | Q] and the place of every entry of Q^T in them
+      std::vector<int> mOff(M.n + 1), mCol(M.col.size() + S.qCol.size());
+#pragma omp parallel for schedule(static)
+      for (int i = 0; i <= M.n; ++i) {
+        mOff[i] = M.off[i] + S.qOff[i];
+        if (i == M.n) continue;
+        int o = mOff[i];
+        for (int e = M.off[i]; e < M.off[i + 1]; ++e) mCol[o++] = M.col[e];
+        for (int e = S.qOff[i]; e < S.qOff[i + 1]; ++e) mCol[o++] = M.n + S.qCol[e];
+      }
+#pragma omp parallel for schedule(static)
+      for (size_t e = 0; e < S.qtSrc.size(); ++e) S.qtSrc[e] += M.off[S.qtCol[e] + 1];
+      f.mOff = ar.upload(mOff);
+      f.mCol = ar.upload(mCol);
+      f.mVal = ar.alloc<T>(mCol.size());
       f.tOff = ar.upload(S.qtOff);
       f.tCol = ar.upload(S.qtCol);
       f.tSrc = ar.upload(S.qtSrc);
       f.nT = (int)S.qtCol.size();
-      f.lanesUp = sa_lanes((long long)M.col.size() + (long long)S.qCol.size(), M.n);
+      f.x = ar.alloc<T>((size_t)M.n + nc);  // [x | the next level's solution]
+      f.lanesUp = sa_lanes((long long)mCol.size(), M.n);
     }
     f.tVal = ar.alloc<T>(f.nT);
-    f.lanesDown = sa_lanes(f.nT, nc);
+    f.lanesDown = nc <= 1024 && f.nT >= 128LL * nc ? kBlock : sa_lanes(f.nT, nc);
     k.n = nc;
     k.rowOff = ar.upload(S.cOff);
     k.col = ar.upload(S.cCol);
@@ -553,8 +568,7 @@ bool build_sa(anb_ctx* c, AmgDevT<T>& A, DevArena& ar, T* val0, T* diag0, T* wdi
     k.diag = ar.alloc<T>(nc);
     k.wdinv = ar.alloc<T>(nc);
     k.b = ar.alloc<T>(nc);
-    k.x = ar.alloc<T>(nc);
-    k.x2 = ar.alloc<T>(nc);
+    k.x2 = l == 0 ? ar.alloc<T>(nc) : f.x + M.n;
     // the uploads' last DMA may still be under way, and the context's stream does not wait for them
     CK(cudaStreamSynchronize(cudaStreamLegacy));
     if (qColS) launch_sa_sell_cols(c->lc, M.n, f.qOff, f.qCol, f.qSlice, qColS);

@@ -349,12 +349,14 @@ struct AmgLevelDevT {
   int maxW;            // level 0: largest SELL slice width
   // smoothed-aggregation hierarchies (AmgDevT::sa) only.  P by rows; A P by rows (the pattern of Q) and
   // Q = (I - w D^-1 A) P, whose values on level 0 are SELL-32 (qSlice, qColS: thread per row) and
-  // elsewhere follow qCol; the restriction operator by coarse rows, gathered from pVal (level 0: P^T)
-  // or qVal (Q^T); P^T for the Galerkin product.
-  const int *pOff, *pCol, *qOff, *qCol, *qSlice, *qColS, *tOff, *tCol, *tSrc, *ptOff, *ptCol, *ptSrc;
-  T *pVal, *apVal, *qVal, *tVal;
+  // elsewhere stand behind the row's -w A in the merged matrix [-w A | Q] (mOff, mCol, mVal; its columns
+  // n + I name the next level's solution, which is stored behind x); the restriction operator by coarse
+  // rows, gathered from pVal (level 0: P^T) or mVal (Q^T); P^T for the Galerkin product.
+  const int *pOff, *pCol, *qOff, *qCol, *qSlice, *qColS, *tOff, *tCol, *tSrc, *ptOff, *ptCol, *ptSrc,
+      *mOff, *mCol;
+  T *pVal, *apVal, *qVal, *tVal, *mVal;
   int nT;              // entries of the restriction operator
-  int lanesDown, lanesUp;  // lanes per row of the restriction from and the up sweep of this level
+  int lanesDown, lanesUp;  // lanes per row of the restriction from (over 32: a block) and the up sweep of this level
   int capQ, capC;      // longest row of Q, and of the next level's matrix + 1
 };
 template <class T>

@@ -11,8 +11,8 @@
 //
 // Against the plain aggregation with over-correction (kernels_krylov.cu) the CG needs half the
 // iterations (143 -> 66 per SIMPLE step on 970k hexes, 151 -> 80 on 334k tets, both to 1e-15) with
-// 11 launches each instead of 17; a step took 30.2 -> 18.5 ms and 13.4 -> 9.8 ms.  An iteration moves
-// 0.5 GB at 970k cells (A twice, Q, P^T, the level-1 matrices) in 185 us: the level-0 kernels run at
+// 11 launches each instead of 17; a step took 30.2 -> 17.5 ms and 13.4 -> 8.7 ms.  An iteration moves
+// 0.5 GB at 970k cells (A twice, Q, P^T, the level-1 matrices) in 170 us: the level-0 kernels run at
 // 3.5-4 TB/s like the other SELL kernels, the levels below 5,000 rows at launch latency.
 #include <algorithm>
 
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kBlock) k_sa_restrict(const int* done, int n, 
     double acc = 0.0;
     if (i < n) {
       const int k1 = __ldg(&off[i + 1]);
-#pragma unroll 4
+#pragma unroll 8
       for (int k = __ldg(&off[i]) + sub; k < k1; k += G) acc += ld(&val[k]) * ld(&x[__ldg(&col[k])]);
     }
     acc = group_sum<G>(acc);
@@ -97,36 +97,49 @@ __global__ void __launch_bounds__(kBlock) k_sa_restrict(const int* done, int n, 
   }
 }
 
-// Up sweep of a coarse level: out = w (b + r1) + Q e, r1 = b - A x with x = w b; G lanes a row.
+// The same with a block a row, for the few long rows of the deep levels (500 rows of 400 entries: a
+// warp a row walks them in 13 dependent steps, 18 us).
+template <class T>
+__global__ void __launch_bounds__(kBlock) k_sa_restrict_block(const int* done, const int* off, const int* col,
+                                                              const T* val, const T* x, T* bNext, const T* w, T* xNext) {
+  __shared__ double sm[32];
+  if (*done) return;
+  const int i = blockIdx.x, k1 = __ldg(&off[i + 1]);
+  double acc[1] = {0.0};
+#pragma unroll 4
+  for (int k = __ldg(&off[i]) + threadIdx.x; k < k1; k += kBlock) acc[0] += ld(&val[k]) * ld(&x[__ldg(&col[k])]);
+  block_reduce<1>(acc, 0u, sm);
+  if (threadIdx.x == 0) {
+    const T b = (T)acc[0];
+    bNext[i] = b;
+    if (w) xNext[i] = (T)(ld(&w[i]) * (double)b);
+  }
+}
+
+// Up sweep of a coarse level: out = x + w r1 + Q e with x = w b and r1 = b - A x, i.e.
+// (2 - omega) x_i + sum of the row [-w_i A_offdiag | Q] times [x | e].  The two matrices are stored as
+// one CSR and the two vectors as one array, so a row is a single gather sum; G lanes a row.
 template <int G, class T>
-__global__ void __launch_bounds__(kBlock) k_sa_up(const int* done, AmgLevelDevT<T> f, const T* e, T* out) {
+__global__ void __launch_bounds__(kBlock) k_sa_up(const int* done, AmgLevelDevT<T> f, double omega, T* out) {
   if (*done) return;
   const int lane = threadIdx.x & 31, sub = lane % G;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nWarps = (gridDim.x * blockDim.x) >> 5;
   for (int base = warp * (32 / G); base < f.n; base += nWarps * (32 / G)) {
     const int i = base + lane / G;
-    double ax = 0.0, qe = 0.0;
+    double y = 0.0;
     if (i < f.n) {
-      const int k0 = __ldg(&f.rowOff[i]), k1 = __ldg(&f.rowOff[i + 1]);
-      const int q0 = __ldg(&f.qOff[i]), q1 = __ldg(&f.qOff[i + 1]);
-#pragma unroll 4
-      for (int k = k0 + sub; k < k1; k += G) ax += ld(&f.val[k]) * ld(&f.x[__ldg(&f.col[k])]);
-#pragma unroll 4
-      for (int k = q0 + sub; k < q1; k += G) qe += ld(&f.qVal[k]) * ld(&e[__ldg(&f.qCol[k])]);
+      const int k1 = __ldg(&f.mOff[i + 1]);
+#pragma unroll 8
+      for (int k = __ldg(&f.mOff[i]) + sub; k < k1; k += G) y += ld(&f.mVal[k]) * ld(&f.x[__ldg(&f.mCol[k])]);
     }
-    ax = group_sum<G>(ax);
-    qe = group_sum<G>(qe);
-    if (i < f.n && sub == 0) {
-      const double b = ld(&f.b[i]), x = ld(&f.x[i]);
-      const double r1 = b - ld(&f.diag[i]) * x - ax;
-      out[i] = (T)(x + ld(&f.wdinv[i]) * r1 + qe);
-    }
+    y = group_sum<G>(y);
+    if (i < f.n && sub == 0) out[i] = (T)((2.0 - omega) * ld(&f.x[i]) + y);
   }
 }
 
 // Up sweep of level 0: z = w (r + r1) + Q e, thread a row over the SELL-32 Q (rows of at most
 // kQChunk entries issue all their loads before the first use), with r.z and beta of the PCG.
-constexpr int kQChunk = 8;
+constexpr int kQChunk = 12;
 template <class T>
 __global__ void __launch_bounds__(kBlock) k_sa_up0(AmgLevelDevT<T> f, const T* e, PcgArgsT<T> a) {
   __shared__ double sm[32];
@@ -188,23 +201,36 @@ struct SaTailArgs {
   int nLev;
   AmgLevelDevT<T> lv[kTailMaxLevels];
   const double* dense;
+  double omega;
 };
 
-template <int G, class T>
-__device__ __forceinline__ void tail_restrict(const AmgLevelDevT<T>& f, const AmgLevelDevT<T>& c, bool last, int warp,
-                                              int nWarps) {
-  const int lane = threadIdx.x & 31, sub = lane % G;
-  for (int base = warp * (32 / G); base < c.n; base += nWarps * (32 / G)) {
-    const int i = base + lane / G;
+// Rows of the cluster's CTAs in turn, a team of TS threads of one CTA a row.
+template <int TS, class T>
+__device__ __forceinline__ void tail_restrict(const AmgLevelDevT<T>& f, const AmgLevelDevT<T>& c, bool last, int rank,
+                                              int nCta, double (&sm)[kTailThreads / 32]) {
+  constexpr int kTeams = kTailThreads / TS;
+  const int team = threadIdx.x / TS, tt = threadIdx.x % TS, lane = threadIdx.x & 31;
+  for (int r0 = 0; r0 < c.n; r0 += nCta * kTeams) {  // uniform over the cluster
+    const int i = r0 + team * nCta + rank;
     double acc = 0.0;
     if (i < c.n) {
       const int k1 = __ldg(&f.tOff[i + 1]);
 #pragma unroll 4
-      for (int k = __ldg(&f.tOff[i]) + sub; k < k1; k += G)
+      for (int k = __ldg(&f.tOff[i]) + tt; k < k1; k += TS)
         acc += ld(&f.tVal[k]) * (double)__ldcg(&f.b[__ldg(&f.tCol[k])]);
     }
-    acc = group_sum<G>(acc);
-    if (i < c.n && sub == 0) {
+    acc = warp_sum(acc);
+    if constexpr (TS > 32) {
+      if (lane == 0) sm[threadIdx.x >> 5] = acc;
+      __syncthreads();
+      if (tt == 0) {
+        acc = 0.0;
+#pragma unroll
+        for (int u = 0; u < TS / 32; ++u) acc += sm[(threadIdx.x >> 5) + u];
+      }
+      __syncthreads();
+    }
+    if (i < c.n && tt == 0) {
       const T b = (T)acc;
       c.b[i] = b;
       if (!last) c.x[i] = (T)(ld(&c.wdinv[i]) * (double)b);
@@ -213,25 +239,19 @@ __device__ __forceinline__ void tail_restrict(const AmgLevelDevT<T>& f, const Am
 }
 
 template <int G, class T>
-__device__ __forceinline__ void tail_up(const AmgLevelDevT<T>& f, const T* e, int warp, int nWarps) {
+__device__ __forceinline__ void tail_up(const AmgLevelDevT<T>& f, double omega, int warp, int nWarps) {
   const int lane = threadIdx.x & 31, sub = lane % G;
   for (int base = warp * (32 / G); base < f.n; base += nWarps * (32 / G)) {
     const int i = base + lane / G;
-    double ax = 0.0, qe = 0.0;
+    double y = 0.0;
     if (i < f.n) {
-      const int k0 = __ldg(&f.rowOff[i]), k1 = __ldg(&f.rowOff[i + 1]);
-      const int q0 = __ldg(&f.qOff[i]), q1 = __ldg(&f.qOff[i + 1]);
-#pragma unroll 4
-      for (int k = k0 + sub; k < k1; k += G) ax += ld(&f.val[k]) * (double)__ldcg(&f.x[__ldg(&f.col[k])]);
-#pragma unroll 4
-      for (int k = q0 + sub; k < q1; k += G) qe += ld(&f.qVal[k]) * (double)__ldcg(&e[__ldg(&f.qCol[k])]);
+      const int k1 = __ldg(&f.mOff[i + 1]);
+#pragma unroll 8
+      for (int k = __ldg(&f.mOff[i]) + sub; k < k1; k += G)
+        y += ld(&f.mVal[k]) * (double)__ldcg(&f.x[__ldg(&f.mCol[k])]);
     }
-    ax = group_sum<G>(ax);
-    qe = group_sum<G>(qe);
-    if (i < f.n && sub == 0) {
-      const double b = (double)__ldcg(&f.b[i]), x = (double)__ldcg(&f.x[i]);
-      f.x2[i] = (T)(x + ld(&f.wdinv[i]) * (b - ld(&f.diag[i]) * x - ax) + qe);
-    }
+    y = group_sum<G>(y);
+    if (i < f.n && sub == 0) f.x2[i] = (T)((2.0 - omega) * (double)__ldcg(&f.x[i]) + y);
   }
 }
 
@@ -239,13 +259,15 @@ template <class T>
 __global__ void __launch_bounds__(kTailThreads, 1) k_sa_tail(const int* done, const __grid_constant__ SaTailArgs<T> a) {
   if (*done) return;
   cg::cluster_group cl = cg::this_cluster();
-  const int t = (int)cl.block_rank() * blockDim.x + threadIdx.x;
-  const int warp = t >> 5, nWarps = ((int)cl.num_blocks() * blockDim.x) >> 5;
+  __shared__ double sm[kTailThreads / 32];
+  const int rank = (int)cl.block_rank(), nCta = (int)cl.num_blocks();
+  const int t = rank * blockDim.x + threadIdx.x;
+  const int warp = t >> 5, nWarps = (nCta * blockDim.x) >> 5;
   const int L = a.nLev;
   for (int l = 0; l + 1 < L; ++l) {
     const bool last = l + 2 == L;
-    if (a.lv[l + 1].n > 512) tail_restrict<16>(a.lv[l], a.lv[l + 1], last, warp, nWarps);
-    else tail_restrict<32>(a.lv[l], a.lv[l + 1], last, warp, nWarps);
+    if (a.lv[l + 1].n > 8 * nCta) tail_restrict<32>(a.lv[l], a.lv[l + 1], last, rank, nCta, sm);
+    else tail_restrict<128>(a.lv[l], a.lv[l + 1], last, rank, nCta, sm);
     cl.sync();
   }
   const AmgLevelDevT<T>& d = a.lv[L - 1];
@@ -259,9 +281,8 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_sa_tail(const int* done, co
   }
   for (int l = L - 2; l >= 0; --l) {
     cl.sync();
-    if (a.lv[l].n > 1024) tail_up<8>(a.lv[l], a.lv[l + 1].x2, warp, nWarps);
-    else if (a.lv[l].n > 512) tail_up<16>(a.lv[l], a.lv[l + 1].x2, warp, nWarps);
-    else tail_up<32>(a.lv[l], a.lv[l + 1].x2, warp, nWarps);
+    if (a.lv[l].n > 32 * nCta) tail_up<16>(a.lv[l], a.omega, warp, nWarps);
+    else tail_up<32>(a.lv[l], a.omega, warp, nWarps);
   }
 }
 
@@ -414,8 +435,9 @@ __global__ void __launch_bounds__(kBlock) k_sa_product(AmgLevelDevT<T> f, AmgLev
       double p = 0.0;
       for (int k = __ldg(&f.pOff[r]); k < __ldg(&f.pOff[r + 1]); ++k)
         if (__ldg(&f.pCol[k]) == J) p = ld(&f.pVal[k]);
-      const int dst = f.qSlice ? __ldg(&f.qSlice[r >> 5]) + (s << 5) + (r & 31) : c0 + s;
-      f.qVal[dst] = (T)(p - ld(&f.wdinv[r]) * sum);
+      const T q = (T)(p - ld(&f.wdinv[r]) * sum);
+      if (f.qSlice) f.qVal[__ldg(&f.qSlice[r >> 5]) + (s << 5) + (r & 31)] = q;
+      else f.mVal[__ldg(&f.rowOff[r + 1]) + c0 + s] = q;  // behind the row's -w A
     } else if (s < nc) {
       c.val[c0 + s] = (T)sum;
     } else {
@@ -431,6 +453,17 @@ __global__ void __launch_bounds__(kBlock) k_sa_sell_cols(int n, const int* off, 
     const int k0 = off[i], k1 = off[i + 1], b = slice[i >> 5] + (i & 31);
     for (int k = k0; k < k1; ++k) out[b + ((k - k0) << 5)] = col[k];
   }
+}
+
+// The -w A part of the merged rows of a coarse level, G lanes a row.
+template <int G, class T>
+__global__ void __launch_bounds__(kBlock) k_sa_scale(AmgLevelDevT<T> f) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = t / G, sub = t % G;
+  if (i >= f.n) return;
+  const double w = ld(&f.wdinv[i]);
+  const int k0 = __ldg(&f.rowOff[i]), k1 = __ldg(&f.rowOff[i + 1]), m0 = __ldg(&f.mOff[i]);
+  for (int k = k0 + sub; k < k1; k += G) f.mVal[m0 + k - k0] = (T)(-w * ld(&f.val[k]));
 }
 
 template <class T>
@@ -537,7 +570,11 @@ void sa_refresh_level(const LaunchCfg& lc, AmgDevT<T>& amg, int l) {
   } else {
     launch_product<8, 256, true>(lc, f, c, amg.omega, f.capQ);
   }
-  k_sa_gather<T><<<grid_for(f.nT, 1 << 30), kBlock, 0, lc.stream>>>(f.nT, f.tSrc, l == 0 ? f.pVal : f.qVal, f.tVal);
+  k_sa_gather<T><<<grid_for(f.nT, 1 << 30), kBlock, 0, lc.stream>>>(f.nT, f.tSrc, l == 0 ? f.pVal : f.mVal, f.tVal);
+  if (l > 0) {
+    g_launches += 1;
+    k_sa_scale<8, T><<<grid_for(8LL * f.n, 1 << 30), kBlock, 0, lc.stream>>>(f);
+  }
   if (sa_small_team(c.n, f.capC)) launch_product<8, 32, false>(lc, f, c, amg.omega, f.capC);
   else launch_product<16, 256, false>(lc, f, c, amg.omega, f.capC);
 }
@@ -560,6 +597,11 @@ void sa_vcycle(const LaunchCfg& lc, const PcgArgsT<T>& a, const AmgDevT<T>* amg,
   auto restrict_to = [&](const AmgLevelDevT<T>& f, const T* x, int l) {
     const AmgLevelDevT<T>& c = amg->lv[l];
     const bool last = l == L - 1;
+    if (f.lanesDown > 32) {
+      k_sa_restrict_block<T><<<c.n, kBlock, 0, lc.stream>>>(a.fl, f.tOff, f.tCol, f.tVal, x, c.b,
+                                                            last ? nullptr : c.wdinv, c.x);
+      return;
+    }
     with_lanes(f.lanesDown, [&](auto G) {
       k_sa_restrict<G.value, T><<<grid_for((long long)G.value * c.n, cap), kBlock, 0, lc.stream>>>(
           a.fl, c.n, f.tOff, f.tCol, f.tVal, x, c.b, last ? nullptr : c.wdinv, c.x);
@@ -581,6 +623,7 @@ void sa_vcycle(const LaunchCfg& lc, const PcgArgsT<T>& a, const AmgDevT<T>* amg,
       ta.nLev = L - t0;
       for (int l = 0; l < ta.nLev; ++l) ta.lv[l] = amg->lv[t0 + l];
       ta.dense = amg->dense;
+      ta.omega = amg->omega;
       cudaLaunchAttribute at[1];
       const cudaLaunchConfig_t cfg = tail_config(lc.stream, amg->tailCluster, at);
       cudaLaunchKernelEx(&cfg, k_sa_tail<T>, (const int*)a.fl, ta);
@@ -591,8 +634,8 @@ void sa_vcycle(const LaunchCfg& lc, const PcgArgsT<T>& a, const AmgDevT<T>* amg,
     for (int l = t0 - 1; l >= 1; --l) {
       const AmgLevelDevT<T>& f = amg->lv[l];
       with_lanes(f.lanesUp, [&](auto G) {
-        k_sa_up<G.value, T><<<grid_for((long long)G.value * f.n, cap), kBlock, 0, lc.stream>>>(a.fl, f,
-                                                                                              amg->lv[l + 1].x2, f.x2);
+        k_sa_up<G.value, T><<<grid_for((long long)G.value * f.n, cap), kBlock, 0, lc.stream>>>(a.fl, f, amg->omega,
+                                                                                              f.x2);
       });
     }
   }
