@@ -456,7 +456,85 @@ int sa_lanes(long long entries, int rows) {
   return g;
 }
 
-// Smoothed-aggregation hierarchy of the current level-0 matrix: patterns on the host, values level
+// The patterns of a level step on the device.  False: a row did not fit the kernels' tables.
+bool sa_pattern_device(anb_ctx* c, DevArena& ar, SaDevPattern& p, bool wantQT) {
+  const LaunchCfg& lc = c->lc;
+  int* info = ar.alloc<int>(16);  // flag, then (total, largest) per scan
+  int* cnt = ar.alloc<int>(std::max(p.n, p.nc));
+  int* cur = ar.alloc<int>(p.nc);
+  CK(cudaMemsetAsync(info, 0, 16 * sizeof(int), c->stream));
+  auto transposed = [&](int entries, const int* off, const int* col, int*& tOff, int* scan) {
+    tOff = ar.alloc<int>((size_t)p.nc + 1);
+    CK(cudaMemsetAsync(cur, 0, sizeof(int) * p.nc, c->stream));
+    sa_count_cols(lc, entries, col, cur);
+    sa_scan(lc, p.nc, cur, tOff, scan);
+  };
+  p.pOff = ar.alloc<int>((size_t)p.n + 1);
+  sa_pattern_rows(lc, p, 0, false, cnt, info);
+  sa_scan(lc, p.n, cnt, p.pOff, info + 2);
+  poll(c, info, 4);
+  if (c->hFlags[0]) return false;
+  p.nP = c->hFlags[2];
+  p.pCol = ar.alloc<int>(p.nP);
+  sa_pattern_rows(lc, p, 0, true, cnt, info);
+  transposed(p.nP, p.pOff, p.pCol, p.ptOff, info + 4);
+  p.qOff = ar.alloc<int>((size_t)p.n + 1);
+  sa_pattern_rows(lc, p, 1, false, cnt, info);
+  sa_scan(lc, p.n, cnt, p.qOff, info + 6);
+  poll(c, info, 8);
+  if (c->hFlags[0]) return false;
+  p.nQ = c->hFlags[6];
+  p.capQ = c->hFlags[7];
+  p.ptCol = ar.alloc<int>(p.nP);
+  p.ptSrc = ar.alloc<int>(p.nP);
+  if (!sa_transpose(lc, p.n, p.nc, c->hFlags[5], p.pOff, p.pCol, p.ptOff, cur, p.ptCol, p.ptSrc)) return false;
+  p.qCol = ar.alloc<int>(p.nQ);
+  sa_pattern_rows(lc, p, 1, true, cnt, info);
+  if (wantQT) transposed(p.nQ, p.qOff, p.qCol, p.qtOff, info + 8);
+  p.cOff = ar.alloc<int>((size_t)p.nc + 1);
+  sa_pattern_rows(lc, p, 2, false, cnt, info);
+  sa_scan(lc, p.nc, cnt, p.cOff, info + 10);
+  poll(c, info, 12);
+  if (c->hFlags[0]) return false;
+  p.nC = c->hFlags[10];
+  p.capC = c->hFlags[11] + 1;
+  p.cCol = ar.alloc<int>(p.nC);
+  sa_pattern_rows(lc, p, 2, true, cnt, info);
+  if (wantQT) {
+    p.qtCol = ar.alloc<int>(p.nQ);
+    p.qtSrc = ar.alloc<int>(p.nQ);
+    if (!sa_transpose(lc, p.n, p.nc, c->hFlags[9], p.qOff, p.qCol, p.qtOff, cur, p.qtCol, p.qtSrc)) return false;
+  }
+  return true;
+}
+
+// The same from the host (sa_setup.cpp), uploaded.
+void sa_pattern_host(DevArena& ar, const SaMatrix& M, const std::vector<int>& agg, SaDevPattern& p, bool wantQT) {
+  const SaPattern S = sa_pattern(M, agg, p.nc, wantQT);
+  p.pOff = ar.upload(S.pOff);
+  p.pCol = ar.upload(S.pCol);
+  p.qOff = ar.upload(S.qOff);
+  p.qCol = ar.upload(S.qCol);
+  p.ptOff = ar.upload(S.ptOff);
+  p.ptCol = ar.upload(S.ptCol);
+  p.ptSrc = ar.upload(S.ptSrc);
+  p.cOff = ar.upload(S.cOff);
+  p.cCol = ar.upload(S.cCol);
+  if (wantQT) {
+    p.qtOff = ar.upload(S.qtOff);
+    p.qtCol = ar.upload(S.qtCol);
+    p.qtSrc = ar.upload(S.qtSrc);
+  }
+  p.nP = (int)S.pCol.size();
+  p.nQ = (int)S.qCol.size();
+  p.nC = (int)S.cCol.size();
+  p.capQ = p.capC = 1;
+  for (int i = 0; i < p.n; ++i) p.capQ = std::max(p.capQ, S.qOff[i + 1] - S.qOff[i]);
+  for (int I = 0; I < p.nc; ++I) p.capC = std::max(p.capC, S.cOff[I + 1] - S.cOff[I] + 1);
+  CK(cudaStreamSynchronize(cudaStreamLegacy));  // the last DMA, before the context's stream reads them
+}
+
+// Smoothed-aggregation hierarchy of the current level-0 matrix: aggregates on the host, patterns, values level
 // by level on the device (the next level's strong couplings come from them).  Returns false, with
 // nothing kept, when the coarsening stalls above the dense solver's size.
 template <class T>
@@ -491,95 +569,91 @@ bool build_sa(anb_ctx* c, AmgDevT<T>& A, DevArena& ar, T* val0, T* diag0, T* wdi
     // Where the next matrix would grow dense (or have a row too long for a block's shared memory),
     // half the threshold is tried: fewer weak couplings, larger aggregates.
     double theta = sa_theta(l, M.n, c->L.maxRowLen);
-    SaPattern S;
+    SaDevPattern p;
     int nc = 0;
     AmgLevelDevT<T>& f = A.lv[l];
     for (int tries = 0;; ++tries, theta *= 0.5) {
-      std::vector<int> agg = sa_aggregate(M, theta, nc);
+      const std::vector<int> agg = sa_aggregate(M, theta, nc);
       if (nc < 1 || nc > (int)(0.9 * M.n)) return reset(false);
       if (tries < 3 && sa_next_entries(M, agg, nc) > 1.25 * M.col.size()) continue;
-      S = sa_pattern(M, std::move(agg), nc, l > 0);
-      f.capQ = f.capC = 1;
-      for (int i = 0; i < M.n; ++i) f.capQ = std::max(f.capQ, S.qOff[i + 1] - S.qOff[i]);
-      for (int I = 0; I < nc; ++I) f.capC = std::max(f.capC, S.cOff[I + 1] - S.cOff[I] + 1);
-      const bool fits = sa_product_smem(8, 256, std::max(f.capQ, f.capC)) <= kSaSmemMax;
-      if (fits) break;
+      p = SaDevPattern{};
+      p.n = M.n;
+      p.nc = nc;
+      p.sliceOff = f.sliceOff;
+      p.rowOff = f.rowOff;
+      p.col = f.col;
+      p.agg = ar.upload(agg);
+      CK(cudaStreamSynchronize(cudaStreamLegacy));  // its last DMA
+      if (!sa_pattern_device(c, ar, p, l > 0)) sa_pattern_host(ar, M, agg, p, l > 0);
+      if (sa_product_smem(8, 256, std::max(p.capQ, p.capC)) <= kSaSmemMax) break;
       if (tries == 3) return reset(false);
     }
     AmgLevelDevT<T>& k = A.lv[l + 1];
     k = AmgLevelDevT<T>{};
     f.nc = nc;
-    f.agg = ar.upload(S.agg);
-    f.pOff = ar.upload(S.pOff);
-    f.pCol = ar.upload(S.pCol);
-    f.pVal = ar.alloc<T>(S.pCol.size());
-    f.qOff = ar.upload(S.qOff);
-    f.qCol = ar.upload(S.qCol);
-    f.apVal = ar.alloc<T>(S.qCol.size());
-    f.ptOff = ar.upload(S.ptOff);
-    f.ptCol = ar.upload(S.ptCol);
-    f.ptSrc = ar.upload(S.ptSrc);
-    int* qColS = nullptr;
+    f.capQ = p.capQ;
+    f.capC = p.capC;
+    f.agg = p.agg;
+    f.pOff = p.pOff;
+    f.pCol = p.pCol;
+    f.pVal = ar.alloc<T>(p.nP);
+    f.qOff = p.qOff;
+    f.qCol = p.qCol;
+    f.apVal = ar.alloc<T>(p.nQ);
+    f.ptOff = p.ptOff;
+    f.ptCol = p.ptCol;
+    f.ptSrc = p.ptSrc;
     if (l == 0) {  // Q in SELL-32 (padding is never read)
       const int nSl = (M.n + kSlice - 1) / kSlice;
-      std::vector<int> sl(nSl + 1, 0);
-      for (int s = 0; s < nSl; ++s) {
-        int w = 0;
-        for (int i = s * kSlice; i < std::min(M.n, (s + 1) * kSlice); ++i) w = std::max(w, S.qOff[i + 1] - S.qOff[i]);
-        sl[s + 1] = sl[s] + w * kSlice;
-      }
-      f.qSlice = ar.upload(sl);
-      qColS = ar.alloc<int>(sl[nSl]);
-      f.qColS = qColS;
-      f.qVal = ar.alloc<T>(sl[nSl]);
-      f.tOff = f.ptOff;
-      f.tCol = f.ptCol;
-      f.tSrc = f.ptSrc;
-      f.nT = (int)S.ptCol.size();
+      int *w = ar.alloc<int>(nSl), *sl = ar.alloc<int>(nSl + 1), *info = ar.alloc<int>(2);
+      sa_slice_widths(c->lc, M.n, p.qOff, w);
+      sa_scan(c->lc, nSl, w, sl, info);
+      poll(c, info, 2);
+      const int slots = c->hFlags[0];
+      int* cs = ar.alloc<int>(slots);
+      launch_sa_sell_cols(c->lc, M.n, p.qOff, p.qCol, sl, cs);
+      f.qSlice = sl;
+      f.qColS = cs;
+      f.qVal = ar.alloc<T>(slots);
+      f.tOff = p.ptOff;
+      f.tCol = p.ptCol;
+      f.tSrc = p.ptSrc;
+      f.nT = p.nP;
     } else {
       // merged rows [-w A | Q] and the place of every entry of Q^T in them
-      std::vector<int> mOff(M.n + 1), mCol(M.col.size() + S.qCol.size());
-#pragma omp parallel for schedule(static)
-      for (int i = 0; i <= M.n; ++i) {
-        mOff[i] = M.off[i] + S.qOff[i];
-        if (i == M.n) continue;
-        int o = mOff[i];
-        for (int e = M.off[i]; e < M.off[i + 1]; ++e) mCol[o++] = M.col[e];
-        for (int e = S.qOff[i]; e < S.qOff[i + 1]; ++e) mCol[o++] = M.n + S.qCol[e];
-      }
-#pragma omp parallel for schedule(static)
-      for (size_t e = 0; e < S.qtSrc.size(); ++e) S.qtSrc[e] += M.off[S.qtCol[e] + 1];
-      f.mOff = ar.upload(mOff);
-      f.mCol = ar.upload(mCol);
-      f.mVal = ar.alloc<T>(mCol.size());
-      f.tOff = ar.upload(S.qtOff);
-      f.tCol = ar.upload(S.qtCol);
-      f.tSrc = ar.upload(S.qtSrc);
-      f.nT = (int)S.qtCol.size();
+      const size_t entries = M.col.size() + (size_t)p.nQ;
+      int *mOff = ar.alloc<int>((size_t)M.n + 1), *mCol = ar.alloc<int>(entries);
+      sa_merge(c->lc, p, mOff, mCol);
+      f.mOff = mOff;
+      f.mCol = mCol;
+      f.mVal = ar.alloc<T>(entries);
+      f.tOff = p.qtOff;
+      f.tCol = p.qtCol;
+      f.tSrc = p.qtSrc;
+      f.nT = p.nQ;
       f.x = ar.alloc<T>((size_t)M.n + nc);  // [x | the next level's solution]
-      f.lanesUp = sa_lanes((long long)mCol.size(), M.n);
+      f.lanesUp = sa_lanes((long long)entries, M.n);
     }
     f.tVal = ar.alloc<T>(f.nT);
     f.lanesDown = nc <= 1024 && f.nT >= 128LL * nc ? kBlock : sa_lanes(f.nT, nc);
     k.n = nc;
-    k.rowOff = ar.upload(S.cOff);
-    k.col = ar.upload(S.cCol);
-    k.val = ar.alloc<T>(S.cCol.size());
+    k.rowOff = p.cOff;
+    k.col = p.cCol;
+    k.val = ar.alloc<T>(p.nC);
     k.diag = ar.alloc<T>(nc);
     k.wdinv = ar.alloc<T>(nc);
     k.b = ar.alloc<T>(nc);
     k.x2 = l == 0 ? ar.alloc<T>(nc) : f.x + M.n;
-    // the uploads' last DMA may still be under way, and the context's stream does not wait for them
-    CK(cudaStreamSynchronize(cudaStreamLegacy));
-    if (qColS) launch_sa_sell_cols(c->lc, M.n, f.qOff, f.qCol, f.qSlice, qColS);
     sa_refresh_level(c->lc, A, l);
-    std::vector<T> v(S.cCol.size()), dg(nc);
+    std::vector<T> v(p.nC), dg(nc);
     CK(cudaMemcpyAsync(v.data(), k.val, v.size() * sizeof(T), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaMemcpyAsync(dg.data(), k.diag, dg.size() * sizeof(T), cudaMemcpyDeviceToHost, c->stream));
+    M.off.resize((size_t)nc + 1);
+    M.col.resize(p.nC);
+    CK(cudaMemcpyAsync(M.off.data(), p.cOff, sizeof(int) * ((size_t)nc + 1), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(M.col.data(), p.cCol, sizeof(int) * p.nC, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     M.n = nc;
-    M.off = S.cOff;
-    M.col = S.cCol;
     M.val.assign(v.begin(), v.end());
     M.diag.assign(dg.begin(), dg.end());
     ++l;

@@ -419,6 +419,26 @@ inline size_t sa_product_smem(int G, int TS, int cap) {
   return (size_t)(kBlock / TS) * cap * ((size_t)(TS / G) * sizeof(double) + sizeof(int));
 }
 inline bool sa_small_team(int rows, int cap) { return rows >= 16384 && sa_product_smem(4, 32, cap) <= kSaSmemMax; }
+// Patterns of a level step on the device (kernels_sa_setup.cu); all arrays on the device.
+struct SaDevPattern {
+  int n = 0, nc = 0;
+  const int *sliceOff = nullptr, *rowOff = nullptr, *col = nullptr;  // the level's matrix (SELL-32 or CSR)
+  const int* agg = nullptr;
+  int *pOff = nullptr, *pCol = nullptr, *qOff = nullptr, *qCol = nullptr, *cOff = nullptr, *cCol = nullptr;
+  int *ptOff = nullptr, *ptCol = nullptr, *ptSrc = nullptr, *qtOff = nullptr, *qtCol = nullptr, *qtSrc = nullptr;
+  int nP = 0, nQ = 0, nC = 0, capQ = 0, capC = 0;  // entries; longest rows of Q and of the next matrix
+};
+// mode 0: P, 1: Q, 2: next matrix.  Row lengths into cnt, or (fill) the columns; *flag: a row did not fit.
+void sa_pattern_rows(const LaunchCfg& lc, const SaDevPattern& p, int mode, bool fill, int* cnt, int* flag);
+// off[0..n] = exclusive scan of cnt; info[0] the total, info[1] the largest
+void sa_scan(const LaunchCfg& lc, int n, const int* cnt, int* off, int* info);
+void sa_count_cols(const LaunchCfg& lc, int entries, const int* col, int* cnt);
+// Transposed rows in ascending order of the original row; false (nothing done): a row is too long.
+bool sa_transpose(const LaunchCfg& lc, int n, int nc, int longest, const int* off, const int* col, const int* tOff,
+                  int* cursor, int* tCol, int* tSrc);
+void sa_slice_widths(const LaunchCfg& lc, int n, const int* off, int* cnt);
+// Merged rows [A | Q] of a coarse level, and Q^T's sources moved to them.
+void sa_merge(const LaunchCfg& lc, const SaDevPattern& p, int* mOff, int* mCol);
 // Columns of a CSR pattern in SELL-32 order (slice offsets given).
 void launch_sa_sell_cols(const LaunchCfg& lc, int n, const int* off, const int* col, const int* slice, int* out);
 template <class T>

@@ -1,4 +1,4 @@
-// Host structure set-up of the smoothed-aggregation hierarchy that preconditions the pressure CG.
+// Host side of the set-up of the smoothed-aggregation hierarchy that preconditions the pressure CG.
 //
 // One level step: strong couplings (a_ij < 0, a_ij^2 > theta^2 a_ii a_jj) give star aggregates (a
 // root with all its strong neighbours where all of them are free; the rows left over join the
