@@ -22,6 +22,8 @@
 //
 // Every kernel is a cell-centric gather over the SELL-32 slots and the cell's boundary faces;
 // face terms needed by both cells of a face are recomputed by each, so there are no atomics.
+#include <algorithm>
+
 #include "kernels.cuh"
 
 namespace anb {
@@ -706,6 +708,12 @@ __global__ void k_count_prec(const int* mom, const int* pres, int* cnt) {
 }  // namespace
 
 static int blocks(const LaunchCfg& lc) { return lc.rowBlocks; }
+// Vectors of 4 nCells entries without a reduction: an entry a thread up to eight blocks an SM (lc.rowBlocks
+// is made for nCells rows, which left the basis updates at 36k cells with four entries a thread: 15 us).
+static int vec_blocks(const LaunchCfg& lc, size_t n) {
+  const size_t cap = 8 * (size_t)std::max(lc.nSM, 148);
+  return (int)std::max<size_t>(1, std::min(cap, (n + kBlock - 1) / kBlock));
+}
 
 void adj_base(const LaunchCfg& lc, const DMesh& m, const AdjArgs& a) {
   g_launches += 1;
@@ -761,15 +769,15 @@ void vec_mdot(const LaunchCfg& lc, size_t n, int k, const double* V, size_t ld, 
 void vec_lincomb(const LaunchCfg& lc, size_t n, int k, const double* V, size_t ld, const double* coef, double sgn,
                  double beta, double* x) {
   g_launches += 1;
-  k_lincomb<<<blocks(lc), kBlock, 0, lc.stream>>>(n, k, V, ld, coef, sgn, beta, x);
+  k_lincomb<<<vec_blocks(lc, n), kBlock, 0, lc.stream>>>(n, k, V, ld, coef, sgn, beta, x);
 }
 void vec_axpby(const LaunchCfg& lc, size_t n, double a, const double* x, double b, double* y) {
   g_launches += 1;
-  k_axpby<<<blocks(lc), kBlock, 0, lc.stream>>>(n, a, x, b, y);
+  k_axpby<<<vec_blocks(lc, n), kBlock, 0, lc.stream>>>(n, a, x, b, y);
 }
 void vec_unit(const LaunchCfg& lc, size_t n, const double* sq, double* x) {
   g_launches += 1;
-  k_unit<<<blocks(lc), kBlock, 0, lc.stream>>>(n, sq, x);
+  k_unit<<<vec_blocks(lc, n), kBlock, 0, lc.stream>>>(n, sq, x);
 }
 void adj_count_prec(const LaunchCfg& lc, const int* mom, const int* pres, int* cnt) {
   g_launches += 1;
