@@ -660,6 +660,12 @@ bool build_sa(anb_ctx* c, AmgDevT<T>& A, DevArena& ar, T* val0, T* diag0, T* wdi
   }
   A.nLevels = l + 1;
   A.sa = 1;
+  const char* verbose = std::getenv("ANB_AMG_VERBOSE");
+  if (verbose && verbose[0] == '1') {
+    std::fprintf(stderr, "AMG levels, smoothed aggregation (rows/longest row of Q/of the next matrix):");
+    for (int q = 0; q < A.nLevels; ++q) std::fprintf(stderr, " %d/%d/%d", A.lv[q].n, A.lv[q].capQ, A.lv[q].capC);
+    std::fprintf(stderr, "\n");
+  }
   A.nDense = M.n;
   A.dense = ar.alloc<double>((size_t)M.n * M.n);
   return true;
@@ -1062,6 +1068,8 @@ int simple_step(anb_ctx* c, anb_iter_stats* st) {
   const int every = std::max(p.p_amg_rebuild_every, 1);
   const bool perSolve = p.p_amg_setup_scope == 1;
   if (perSolve || !c->amgBuilt || c->outerStep == 1 || ((c->outerStep - 1) % every) == 0) ensure_amg(c);
+  else if (p.p_use_amg && c->mixed && c->amg32.sa) sa_refresh_fine(c->lc, c->amg32);
+  else if (p.p_use_amg && c->amg.sa) sa_refresh_fine(c->lc, c->amg);
   // 4. non-orthogonal pressure passes
   const int nPS = std::max(p.n_nonorth_corr, 0) + 1, nExtra = std::max(p.n_pressure_corr, 0);
   const int total = nPS + nExtra;

@@ -412,6 +412,9 @@ template <class T>
 void sa_refresh_level(const LaunchCfg& lc, AmgDevT<T>& amg, int l);
 template <class T>
 void sa_refresh(const LaunchCfg& lc, AmgDevT<T>& amg);
+// Only the finest Q, for a matrix that changed under a hierarchy that is kept.
+template <class T>
+void sa_refresh_fine(const LaunchCfg& lc, AmgDevT<T>& amg);
 // Dynamic shared memory of one block of the refresh's sparse products, and whether a row of the product
 // goes to one warp (many rows) or to a whole block.
 constexpr size_t kSaSmemMax = 200 * 1024;

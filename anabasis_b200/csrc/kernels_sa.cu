@@ -550,15 +550,11 @@ static void launch_product(const LaunchCfg& lc, const AmgLevelDevT<T>& f, const 
   kern<<<(rows + kTeams - 1) / kTeams, kBlock, smem, lc.stream>>>(f, c, omega, cap);
 }
 
+// A P and Q of level l from the stored P
 template <class T>
-void sa_refresh_level(const LaunchCfg& lc, AmgDevT<T>& amg, int l) {
+static void refresh_q(const LaunchCfg& lc, AmgDevT<T>& amg, int l) {
   AmgLevelDevT<T>& f = amg.lv[l];
   AmgLevelDevT<T>& c = amg.lv[l + 1];
-  g_launches += 4;
-  if (l == 0) k_sa_p<1, T><<<(f.n + kBlock - 1) / kBlock, kBlock, 0, lc.stream>>>(f, kSaOmegaP);
-  else with_lanes(f.lanesUp, [&](auto G) {
-    k_sa_p<G.value, T><<<grid_for((long long)G.value * f.n, 1 << 30), kBlock, 0, lc.stream>>>(f, kSaOmegaP);
-  });
   // a warp a row while there are rows enough to fill the GPU with warps, else a block a row
   const size_t smem0 = (size_t)f.capQ * kApThreads * (sizeof(double) + sizeof(int));
   if (l == 0 && smem0 <= 96 * 1024) {
@@ -570,6 +566,18 @@ void sa_refresh_level(const LaunchCfg& lc, AmgDevT<T>& amg, int l) {
   } else {
     launch_product<8, 256, true>(lc, f, c, amg.omega, f.capQ);
   }
+}
+
+template <class T>
+void sa_refresh_level(const LaunchCfg& lc, AmgDevT<T>& amg, int l) {
+  AmgLevelDevT<T>& f = amg.lv[l];
+  AmgLevelDevT<T>& c = amg.lv[l + 1];
+  g_launches += 4;
+  if (l == 0) k_sa_p<1, T><<<(f.n + kBlock - 1) / kBlock, kBlock, 0, lc.stream>>>(f, kSaOmegaP);
+  else with_lanes(f.lanesUp, [&](auto G) {
+    k_sa_p<G.value, T><<<grid_for((long long)G.value * f.n, 1 << 30), kBlock, 0, lc.stream>>>(f, kSaOmegaP);
+  });
+  refresh_q(lc, amg, l);
   k_sa_gather<T><<<grid_for(f.nT, 1 << 30), kBlock, 0, lc.stream>>>(f.nT, f.tSrc, l == 0 ? f.pVal : f.mVal, f.tVal);
   if (l > 0) {
     g_launches += 1;
@@ -577,6 +585,15 @@ void sa_refresh_level(const LaunchCfg& lc, AmgDevT<T>& amg, int l) {
   }
   if (sa_small_team(c.n, f.capC)) launch_product<8, 32, false>(lc, f, c, amg.omega, f.capC);
   else launch_product<16, 256, false>(lc, f, c, amg.omega, f.capC);
+}
+
+// With a stale hierarchy (p_amg_rebuild_every > 1) the finest Q still has to belong to the current matrix:
+// the restriction goes through the current residual, and with an older Q the preconditioner would lose its
+// symmetry.  P and the coarse levels stay as they are.
+template <class T>
+void sa_refresh_fine(const LaunchCfg& lc, AmgDevT<T>& amg) {
+  g_launches += 1;
+  refresh_q(lc, amg, 0);
 }
 
 template <class T>
@@ -668,6 +685,7 @@ void sa_configure_tail(AmgDevT<T>& amg, int tailRows, cudaStream_t s) {
 #define ANB_INSTANTIATE(T)                                                          \
   template void sa_refresh_level<T>(const LaunchCfg&, AmgDevT<T>&, int);            \
   template void sa_refresh<T>(const LaunchCfg&, AmgDevT<T>&);                       \
+  template void sa_refresh_fine<T>(const LaunchCfg&, AmgDevT<T>&);                  \
   template void sa_configure_tail<T>(AmgDevT<T>&, int, cudaStream_t);               \
   template void sa_vcycle<T>(const LaunchCfg&, const PcgArgsT<T>&, const AmgDevT<T>*, int);
 ANB_INSTANTIATE(double)

@@ -53,3 +53,25 @@ def test_mixed_precision_fields(kw):
     scale = max(np.abs(out[0][k]).max() for k in "uvw")
     for k in "uvw":
         assert np.abs(out[0][k] - out[1][k]).max() <= 1e-5 * scale, k
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_stale_hierarchy(precision):
+    """Coarse levels kept for four steps under a matrix that changes every step: the preconditioner must stay
+    symmetric (the finest Q follows the matrix), so the fields are those of a refresh every step and the
+    iterations grow mildly.  Both solve to 1e-14: 1e-8 as in test_gpu_parity; a stale V-cycle costs a few
+    iterations a solve, twice the fresh count is the bound."""
+    m, bc, _ = channel(nx=41, ny=16, nz=17, jitter=0.1, seed=2)
+    u, v, w, p = random_state(m, 7)
+    got = []
+    for every in (1, 4):
+        s = anb.Solver(m, anb.default_params(mu=1e-3, u_relax=0.7, p_relax=0.3, vel_tol=1e-14, p_tol=1e-14,
+                                             vel_maxit=2000, precision=precision, p_amg_rebuild_every=every))
+        s.set_bc(bc)
+        s.set_state(0.2 * u, 0.2 * v, 0.2 * w, 0.2 * p)
+        _, st = s.iterate(6)
+        got.append((s.get_state(), sum(x["its_p_total"] for x in st), [x["status"] for x in st]))
+    scale = max(np.abs(got[0][0][k]).max() for k in "uvw")
+    for k in "uvw":
+        assert np.abs(got[0][0][k] - got[1][0][k]).max() <= 1e-8 * scale, k
+    assert got[1][1] <= 2 * got[0][1] and not any(got[1][2]), got
