@@ -3,17 +3,20 @@
 //
 // Up to a few hundred thousand unknowns the five kernels of an iteration move data that stays in L2
 // and cost their launches and the fence-ticket-read chains of their reductions: 27 us an iteration
-// for 3 x 16k unknowns.  Here every thread keeps its rows' vectors (and up to two rows of the matrix)
-// in registers for the whole solve; only D^-1 p and D^-1 s go through memory, because the products
-// gather them, and an iteration is four grid barriers (about 11 us in all), each of which carries the block partials of
-// the sums due there.  All blocks add the partials in the same order, so they take the same branches
-// and the result does not depend on timing.  The grid is one block per SM (cooperative launch); a
-// barrier that is not reached within kSpinLimit polls sets the fail flag and every block returns.
+// for 3 x 16k unknowns.  Here every thread keeps its rows' vectors in registers and its rows of the
+// matrix in registers or shared memory for the whole solve; only D^-1 p and D^-1 s go through memory,
+// because the products gather them, and an iteration is four grid barriers (about 10 us in all), each of
+// which carries the block partials of the sums due there.  All blocks add the partials in the same order,
+// so they take the same branches and the result does not depend on timing.  The grid is one block per SM
+// (cooperative launch); a barrier that is not reached within kSpinLimit polls sets the fail flag and every
+// block returns.
 //
-// Measured (ms per pass, five kernels -> one): SIMPLE steps on 16k hexes 21.4 -> 16.1, 36k with all
-// correctors 22.9 -> 18.6, scalar transport on 262k cells 44 -> 24, force gradient at 36k 88 -> 70.  The
-// line is drawn at four rows a thread (303k unknowns), the last size measured faster: 3 x 91k 4.6 -> 4.2
-// ms a step; beyond it the vectors outgrow the registers and the five kernels are bandwidth-bound.
+// Measured (ms per pass, five kernels -> one): SIMPLE steps on 16k hexes 21.4 -> 15.5, 36k with all
+// correctors 22.9 -> 18.0, scalar transport on 262k cells 44 -> 24, force gradient at 36k 88 -> 70; with
+// the matrix of four rows a thread in shared memory instead of L2, and no fences beyond the release and
+// acquire of the barriers, transport 14.0 -> 10.8.  The line is drawn at four rows a thread (303k
+// unknowns), the last size measured faster (3 x 91k 4.6 -> 4.2 ms a step); beyond it the vectors outgrow
+// the registers.
 #include <algorithm>
 
 #include "krylov_dev.cuh"
@@ -78,13 +81,12 @@ __device__ __forceinline__ bool grid_sum(const CoopBar& bar, CoopShared& sh, uns
   ++epoch;
   __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence();
+    // release and acquire order the whole block's accesses: the block barriers around them are cumulative
     add_release(bar.count);
     const unsigned want = epoch * (unsigned)nb;
     unsigned n = 0;
     while (ld_acquire(bar.count) < want && n < kSpinLimit) ++n;
     sh.bad = n >= kSpinLimit;
-    __threadfence();
   }
   __syncthreads();
   if (sh.bad) {
@@ -103,10 +105,21 @@ __device__ __forceinline__ bool grid_sum(const CoopBar& bar, CoopShared& sh, uns
   return true;
 }
 
-// R rows a thread; WM: bound on the row width (0: any); rows of the matrix in registers when kReg.
-template <int R, int WM, bool kReg>
+// Where a thread keeps its rows of the matrix for the whole solve: one row of registers, shared memory
+// for two and four (12 bytes a slot: at most 196 KB for four rows of eight), memory for wider rows.
+enum class Keep { kRegisters, kShared, kMemory };
+constexpr size_t coop_smem(Keep keep, int R, int WM) {
+  return keep == Keep::kShared ? (size_t)R * WM * kCoopThreads * (sizeof(double) + sizeof(int)) : 0;
+}
+
+// R rows a thread; WM: bound on the row width (0: any).
+template <int R, int WM, Keep kKeep>
 __global__ void __launch_bounds__(kCoopThreads, 1) k_bicg_coop(BicgArgs a, int mask, CoopBar bar) {
+  constexpr bool kReg = kKeep == Keep::kRegisters;
   __shared__ CoopShared sh;
+  extern __shared__ double keep[];  // values [slot][thread], then columns
+  double* sVal = keep + threadIdx.x;
+  int* sCol = reinterpret_cast<int*>(keep + (size_t)R * WM * kCoopThreads) + threadIdx.x;
   const int n = a.A.n, nc = a.nc, lane = threadIdx.x & 31;
   // warps take the components in turn, so that the warps of a block read the same matrix rows
   const int gw = blockIdx.x * kCoopWarps + (threadIdx.x >> 5);
@@ -129,12 +142,12 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_bicg_coop(BicgArgs a, int m
       for (int e = 0; e < WM; ++e) g[e] = __ldcg(&z[col[k][e]]);
 #pragma unroll
       for (int e = 0; e < WM; ++e) y += val[k][e] * g[e];
-    } else if constexpr (WM > 0) {
-      int c[WM];
-      double m[WM];
-      sell_regs<WM>(a.A.sliceOff, a.A.col, a.A.val, row[k], c, m);
+    } else if constexpr (kKeep == Keep::kShared) {
+      double g[WM];
 #pragma unroll
-      for (int e = 0; e < WM; ++e) y += m[e] * __ldcg(&z[c[e]]);
+      for (int e = 0; e < WM; ++e) g[e] = __ldcg(&z[sCol[(k * WM + e) * kCoopThreads]]);
+#pragma unroll
+      for (int e = 0; e < WM; ++e) y += sVal[(k * WM + e) * kCoopThreads] * g[e];
     } else {
       const int b = __ldg(&a.A.sliceOff[row[k] >> 5]) + (row[k] & 31);
       const int W = (__ldg(&a.A.sliceOff[(row[k] >> 5) + 1]) - __ldg(&a.A.sliceOff[row[k] >> 5])) >> 5;
@@ -160,6 +173,16 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_bicg_coop(BicgArgs a, int m
     }
     if (row[k] < 0) continue;
     if constexpr (kReg) sell_regs<WM>(a.A.sliceOff, a.A.col, a.A.val, i, col[k], val[k]);
+    if constexpr (kKeep == Keep::kShared) {
+      int c[WM];
+      double m[WM];
+      sell_regs<WM>(a.A.sliceOff, a.A.col, a.A.val, i, c, m);
+#pragma unroll
+      for (int e = 0; e < WM; ++e) {
+        sCol[(k * WM + e) * kCoopThreads] = c[e];
+        sVal[(k * WM + e) * kCoopThreads] = m[e];
+      }
+    }
     dg[k] = ld(&a.A.diag[i]);
     dinv[k] = 1.0 / dg[k];
     x[k] = a.x[o + i];
@@ -296,14 +319,16 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_bicg_coop(BicgArgs a, int m
   if (blockIdx.x == 0 && threadIdx.x == 0) a.fl[12] = 0;
 }
 
-template <int R, int WM, bool kReg>
+template <int R, int WM, Keep kKeep>
 bool launch_one(cudaStream_t s, int blocks, const BicgArgs& a, int mask, const CoopBar& bar) {
-  auto kern = k_bicg_coop<R, WM, kReg>;
+  auto kern = k_bicg_coop<R, WM, kKeep>;
+  constexpr size_t smem = coop_smem(kKeep, R, WM);
   BicgArgs aa = a;
   int m = mask;
   CoopBar b = bar;
   void* args[] = {&aa, &m, &b};
-  if (cudaLaunchCooperativeKernel((const void*)kern, dim3(blocks), dim3(kCoopThreads), args, 0, s) == cudaSuccess)
+  if ((smem == 0 || cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess) &&
+      cudaLaunchCooperativeKernel((const void*)kern, dim3(blocks), dim3(kCoopThreads), args, smem, s) == cudaSuccess)
     return true;
   cudaGetLastError();
   return false;
@@ -311,9 +336,15 @@ bool launch_one(cudaStream_t s, int blocks, const BicgArgs& a, int mask, const C
 
 template <int WM>
 bool launch_width(cudaStream_t s, int blocks, int rows, const BicgArgs& a, int mask, const CoopBar& bar) {
-  if (rows <= 1) return launch_one<1, WM, (WM > 0)>(s, blocks, a, mask, bar);
-  if (rows <= 2) return launch_one<2, WM, (WM > 0 && WM <= 6)>(s, blocks, a, mask, bar);
-  return launch_one<4, WM, false>(s, blocks, a, mask, bar);
+  if constexpr (WM == 0) {
+    if (rows <= 1) return launch_one<1, 0, Keep::kMemory>(s, blocks, a, mask, bar);
+    if (rows <= 2) return launch_one<2, 0, Keep::kMemory>(s, blocks, a, mask, bar);
+    return launch_one<4, 0, Keep::kMemory>(s, blocks, a, mask, bar);
+  } else {
+    if (rows <= 1) return launch_one<1, WM, Keep::kRegisters>(s, blocks, a, mask, bar);
+    if (rows <= 2) return launch_one<2, WM, Keep::kShared>(s, blocks, a, mask, bar);
+    return launch_one<4, WM, Keep::kShared>(s, blocks, a, mask, bar);
+  }
 }
 
 }  // namespace
