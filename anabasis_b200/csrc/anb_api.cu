@@ -531,7 +531,6 @@ void sa_pattern_host(DevArena& ar, const SaMatrix& M, const std::vector<int>& ag
   p.capQ = p.capC = 1;
   for (int i = 0; i < p.n; ++i) p.capQ = std::max(p.capQ, S.qOff[i + 1] - S.qOff[i]);
   for (int I = 0; I < p.nc; ++I) p.capC = std::max(p.capC, S.cOff[I + 1] - S.cOff[I] + 1);
-  CK(cudaStreamSynchronize(cudaStreamLegacy));  // the last DMA, before the context's stream reads them
 }
 
 // Smoothed-aggregation hierarchy of the current level-0 matrix: aggregates on the host, patterns, values level
@@ -583,7 +582,6 @@ bool build_sa(anb_ctx* c, AmgDevT<T>& A, DevArena& ar, T* val0, T* diag0, T* wdi
       p.rowOff = f.rowOff;
       p.col = f.col;
       p.agg = ar.upload(agg);
-      CK(cudaStreamSynchronize(cudaStreamLegacy));  // its last DMA
       if (!sa_pattern_device(c, ar, p, l > 0)) sa_pattern_host(ar, M, agg, p, l > 0);
       if (sa_product_smem(8, 256, std::max(p.capQ, p.capC)) <= kSaSmemMax) break;
       if (tries == 3) return reset(false);
@@ -759,7 +757,6 @@ void build_amg(anb_ctx* c, AmgDevT<T>& A, std::vector<AmgLevelHost>& H, DevArena
   A.nDense = nd;
   A.dense = ar.alloc<double>((size_t)nd * nd);
   if (ga) c->amgBuilt = true;
-  CK(cudaStreamSynchronize(cudaStreamLegacy));  // the uploads, before the context's stream reads them
   const char* tailEnv = std::getenv("ANB_AMG_TAIL_ROWS");
   amg_configure_tail(A, tailEnv ? std::atoi(tailEnv) : kAmgTailRows, c->stream);
   const char* fdEnv = std::getenv("ANB_AMG_FUSED_DOWN_ROWS");
@@ -1596,8 +1593,8 @@ int anb_set_bc(anb_ctx* c, const int* tu, const int* tv, const int* tw, const in
       val[(size_t)3 * nB + b] = pf[nI + b];
       if ((ty[b] & 8) && pf[nI + b] != 0.0) pZero = false;
     }
-    CK(cudaMemcpy(c->dBType, ty.data(), nB, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(c->dBVal, val.data(), val.size() * sizeof(double), cudaMemcpyHostToDevice));
+    upload_now(c->dBType, ty.data(), nB);
+    upload_now(c->dBVal, val.data(), val.size() * sizeof(double));
     c->pZeroBC = pZero;
     c->bcSet = true;
     return ANB_OK;
