@@ -643,6 +643,7 @@ bool build_sa(anb_ctx* c, AmgDevT<T>& A, DevArena& ar, T* val0, T* diag0, T* wdi
     k.b = ar.alloc<T>(nc);
     k.x2 = l == 0 ? ar.alloc<T>(nc) : f.x + M.n;
     sa_refresh_level(c->lc, A, l);
+    CK(cudaGetLastError());
     std::vector<T> v(p.nC), dg(nc);
     CK(cudaMemcpyAsync(v.data(), k.val, v.size() * sizeof(T), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaMemcpyAsync(dg.data(), k.diag, dg.size() * sizeof(T), cudaMemcpyDeviceToHost, c->stream));
@@ -808,6 +809,7 @@ void ensure_amg(anb_ctx* c) {
       build_amg<float>(c, c->amg32, c->amgHost, c->amgArena, c->pval32, c->pdiag32, c->pwdinv32, &ga);
     }
     if (c->amg32.nLevels >= 2) amg_refresh(c->lc, c->amg32);
+    CK(cudaGetLastError());
     return;
   }
   if (!c->amgBuilt) {
@@ -815,6 +817,7 @@ void ensure_amg(anb_ctx* c) {
     build_amg<double>(c, c->amg, c->amgHost, c->amgArena, c->pval, c->pdiag, c->pwdinv, &ga);
   }
   if (c->amg.nLevels >= 2) amg_refresh(c->lc, c->amg);
+  CK(cudaGetLastError());
 }
 
 constexpr int kScalDefect = 32;  // 3 * 8

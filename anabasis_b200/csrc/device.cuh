@@ -10,6 +10,14 @@ namespace anb {
 constexpr int kBlock = 256;
 constexpr int kWarp = 32;
 
+// Lets a kernel be launched with up to kBytes of dynamic shared memory.  The limit belongs to the function on
+// the device, which every context and thread of the process shares: it is a constant of the kernel, never the
+// need of one launch, or a thread could lower it between another's call and its launch.
+template <size_t kBytes, class K>
+cudaError_t allow_smem(K* kern) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBytes);
+}
+
 // One internal face, 64 bytes: two 32-byte sectors per gather.
 struct __align__(16) FaceRec {
   double lam;     // clamped weight toward the neighbour (new orientation)

@@ -327,7 +327,7 @@ bool launch_one(cudaStream_t s, int blocks, const BicgArgs& a, int mask, const C
   int m = mask;
   CoopBar b = bar;
   void* args[] = {&aa, &m, &b};
-  if ((smem == 0 || cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess) &&
+  if ((smem == 0 || allow_smem<smem>(kern) == cudaSuccess) &&
       cudaLaunchCooperativeKernel((const void*)kern, dim3(blocks), dim3(kCoopThreads), args, smem, s) == cudaSuccess)
     return true;
   cudaGetLastError();

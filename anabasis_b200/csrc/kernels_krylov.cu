@@ -1431,7 +1431,7 @@ void amg_dense_factor(const LaunchCfg& lc, const AmgLevelDevT<T>& c, double* inv
   g_launches += 1;
   const int nc = (c.n + 31) / 32;
   auto go = [&](auto kern) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (allow_smem<200 * 1024>(kern) != cudaSuccess) return;  // cudaGetLastError reports it
     kern<<<1, 1024, smem, lc.stream>>>(c, inv);
   };
   if (nc <= 1) go(k_amg_dense_factor<T, 1>);

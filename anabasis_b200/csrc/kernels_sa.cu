@@ -544,7 +544,7 @@ static void launch_product(const LaunchCfg& lc, const AmgLevelDevT<T>& f, const 
                            int cap) {
   const size_t smem = sa_product_smem(G, TS, cap);
   auto kern = k_sa_product<G, TS, kAP, T>;
-  if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (smem > 48 * 1024 && allow_smem<kSaSmemMax>(kern) != cudaSuccess) return;  // cudaGetLastError reports it
   constexpr int kTeams = kBlock / TS;
   const int rows = kAP ? f.n : c.n;
   kern<<<(rows + kTeams - 1) / kTeams, kBlock, smem, lc.stream>>>(f, c, omega, cap);
@@ -557,9 +557,9 @@ static void refresh_q(const LaunchCfg& lc, AmgDevT<T>& amg, int l) {
   AmgLevelDevT<T>& c = amg.lv[l + 1];
   // a warp a row while there are rows enough to fill the GPU with warps, else a block a row
   const size_t smem0 = (size_t)f.capQ * kApThreads * (sizeof(double) + sizeof(int));
-  if (l == 0 && smem0 <= 96 * 1024) {
-    if (smem0 > 48 * 1024)
-      cudaFuncSetAttribute(k_sa_ap0<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem0);
+  constexpr size_t kAp0Smem = 96 * 1024;
+  if (l == 0 && smem0 <= kAp0Smem) {
+    if (smem0 > 48 * 1024 && allow_smem<kAp0Smem>(k_sa_ap0<T>) != cudaSuccess) return;
     k_sa_ap0<T><<<(f.n + kApThreads - 1) / kApThreads, kApThreads, smem0, lc.stream>>>(f, f.capQ);
   } else if (sa_small_team(f.n, f.capQ)) {
     launch_product<8, 32, true>(lc, f, c, amg.omega, f.capQ);
