@@ -68,8 +68,7 @@ double env_or(const char* name, double dflt) {
 
 AdjointData& adj(anb_ctx* c) {
   if (c->adj) return *c->adj;
-  auto* d = new AdjointData();
-  c->adj = d;
+  auto d = std::make_unique<AdjointData>();  // kept only when every allocation has succeeded
   DevArena& A = d->ar;
   const int C = c->C;
   d->C = C;
@@ -100,7 +99,6 @@ AdjointData& adj(anb_ctx* c) {
   // h of the two Gram-Schmidt passes, the squared norm after them, and the work counters
   d->coef = A.alloc<double>(2 * (size_t)(d->mBasis + 2) + 4);
   d->cnt = reinterpret_cast<int*>(d->coef + 2 * (d->mBasis + 2) + 1);
-  CK(cudaMallocHost(&d->hCoef, sizeof(double) * (2 * (size_t)(d->mBasis + 2) + 4)));
   d->gX = A.alloc<double>(d->N);
   d->R = A.alloc<double>(d->N);
   d->t1 = A.alloc<double>(d->N);
@@ -121,7 +119,9 @@ AdjointData& adj(anb_ctx* c) {
     tw[c->slotNei[f]] = c->slotOwn[f];
   }
   d->twin = A.upload(tw);
-  return *d;
+  CK(cudaMallocHost(&d->hCoef, sizeof(double) * (2 * (size_t)(d->mBasis + 2) + 4)));
+  c->adj = d.release();
+  return *c->adj;
 }
 
 AdjArgs adj_args(anb_ctx* c, AdjointData& d) {

@@ -1685,21 +1685,22 @@ int anb_patch_force(anb_ctx* c, int patch, int sign, anb_force_report* out) {
 namespace {
 
 void ensure_scalar_buffers(anb_ctx* c) {
-  if (c->sPhi) return;
-  DevArena& A = c->scalarArena;
-  const int C = c->C, nF = c->nI + c->nB;
-  c->sMinv = A.alloc<double>((size_t)6 * C);
-  c->sBcType = A.alloc<uint8_t>(c->nB);
-  c->sBcVal = A.alloc<double>(c->nB);
-  c->sGamma = A.alloc<double>(nF);
-  c->sFlux = A.alloc<double>(nF);
-  c->sSrc = A.alloc<double>(C);
-  c->sSp = A.alloc<double>(C);
-  c->sPhi = A.alloc<double>(C);
-  c->sGrad = A.alloc<double>((size_t)3 * C);
-  c->sRaw = A.alloc<double>(nF);
-  c->sOrig = A.upload(c->L.fOrig);
-  c->sFlip = A.upload(c->L.fFlip);
+  build_once(c->scalarReady, c->scalarArena, [&] {
+    DevArena& A = c->scalarArena;
+    const int C = c->C, nF = c->nI + c->nB;
+    c->sMinv = A.alloc<double>((size_t)6 * C);
+    c->sBcType = A.alloc<uint8_t>(c->nB);
+    c->sBcVal = A.alloc<double>(c->nB);
+    c->sGamma = A.alloc<double>(nF);
+    c->sFlux = A.alloc<double>(nF);
+    c->sSrc = A.alloc<double>(C);
+    c->sSp = A.alloc<double>(C);
+    c->sPhi = A.alloc<double>(C);
+    c->sGrad = A.alloc<double>((size_t)3 * C);
+    c->sRaw = A.alloc<double>(nF);
+    c->sOrig = A.upload(c->L.fOrig);
+    c->sFlip = A.upload(c->L.fFlip);
+  });
 }
 
 // Face array in input order/orientation -> device (layout order; fluxes change sign on flipped

@@ -95,6 +95,7 @@ struct anb_ctx {
   double innerRtol = 1e-4;    // relative reduction asked of one FP32 inner solve at most
   // scalar-library solves (allocated on first use)
   DevArena scalarArena;
+  bool scalarReady = false;
   double *sMinv = nullptr, *sBcVal = nullptr, *sGamma = nullptr, *sFlux = nullptr, *sSrc = nullptr,
          *sSp = nullptr, *sPhi = nullptr, *sGrad = nullptr, *sRaw = nullptr;
   int* sOrig = nullptr;

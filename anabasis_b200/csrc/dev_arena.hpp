@@ -83,4 +83,18 @@ class DevArena {
   size_t cur_ = 0, used_ = 0, bytes_ = 0;
 };
 
+// Runs make(), which fills a group of buffers from the arena, unless it is ready.  When an allocation fails
+// half way the arena is given back and the group stays not ready, so that the next use starts afresh.
+template <class F>
+void build_once(bool& ready, DevArena& arena, F&& make) {
+  if (ready) return;
+  try {
+    make();
+  } catch (...) {
+    arena.release();
+    throw;
+  }
+  ready = true;
+}
+
 }  // namespace anb

@@ -72,6 +72,30 @@ int main() {
   if (std::memcmp(d, h.data(), h.size() * sizeof(int))) return fail("an earlier upload was overwritten");
   a.release();
   if (g_held) return fail("release left memory behind");
+
+  // a group of buffers whose second allocation fails: not ready, nothing held, made anew later
+  bool ready = false;
+  const void *first = nullptr, *second = nullptr;
+  auto make = [&] {
+    first = a.alloc<char>((size_t)64 << 20);
+    second = a.alloc<char>((size_t)96 << 20);
+  };
+  g_limit = (size_t)128 << 20;
+  bool threw = false;
+  try {
+    anb::build_once(ready, a, make);
+  } catch (const anb::AnbError& e) {
+    threw = e.code == ANB_ERR_CUDA;
+  }
+  if (!threw || ready || second || g_held) return fail("a failed group was kept");
+  g_limit = ~(size_t)0;
+  first = nullptr;
+  anb::build_once(ready, a, make);
+  if (!ready || !first || !second) return fail("a failed group was not made anew");
+  const void* was = first;
+  anb::build_once(ready, a, make);
+  if (first != was) return fail("a ready group was made twice");
+  a.release();
   std::printf("ok\n");
   return 0;
 }
