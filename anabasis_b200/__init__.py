@@ -110,6 +110,7 @@ SIGNATURES = {
     "anb_debug_momentum": (ct.c_int, [ct.c_void_p, _dp, _dp, _dp, _dp, _dp, _dp, _dp, _dp, _dp]),
     "anb_debug_pressure": (ct.c_int, [ct.c_void_p, _dp, _dp, _dp, _dp, _dp, _dp, _dp, _dp, _dp]),
     "anb_debug_pressure_solve": (ct.c_int, [ct.c_void_p, _dp, _dp, _ip, _dp]),
+    "anb_debug_hierarchy": (ct.c_int, [ct.c_void_p, ct.c_int, ct.c_int, ct.POINTER(ct.c_longlong), _dp]),
     "anb_debug_nonorth": (ct.c_int, [ct.c_void_p, _dp, _dp, _dp, _dp, _dp]),
     "anb_mesh_read_polymesh": (ct.c_int, [ct.c_char_p, ct.POINTER(ct.c_void_p), ct.c_char_p, ct.c_int]),
     "anb_mesh_make_channel": (ct.c_int, [ct.c_int, ct.c_int, ct.c_int, ct.c_double, ct.c_double, ct.c_double,
@@ -442,6 +443,21 @@ class Solver:
         self._check(lib().anb_debug_pressure_solve(self._h, _d(b), _d(x), ct.byref(its), ct.byref(res)),
                     ok=(ANB_OK, ANB_NOT_CONVERGED))
         return x, its.value, res.value
+
+    def debug_hierarchy(self) -> list[dict]:
+        """anb_debug_hierarchy: every array of every level, keyed as in include/anb.h."""
+        keys = ("sizes", "off", "col", "val", "diag", "weight", "agg", "p_off", "p_col", "p_val", "q_off", "q_col",
+                "r_off", "r_col", "r_val")
+
+        def get(level, k):
+            n = ct.c_longlong(0)
+            self._check(lib().anb_debug_hierarchy(self._h, level, k, ct.byref(n), None))
+            a = np.empty(n.value)
+            self._check(lib().anb_debug_hierarchy(self._h, level, k, ct.byref(n), _d(a)))
+            return a if keys[k] in ("val", "diag", "weight", "p_val", "r_val") else a.astype(np.int64)
+
+        levels = int(get(0, 0)[0])
+        return [{keys[k]: get(l, k) for k in range(len(keys) if l + 1 < levels else 6)} for l in range(levels)]
 
     def close(self) -> None:
         if getattr(self, "_h", None) is not None:

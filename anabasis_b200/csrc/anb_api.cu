@@ -2099,6 +2099,60 @@ int anb_debug_pressure_solve(anb_ctx* c, const double* b, double* x, int* iters,
   });
 }
 
+int anb_debug_hierarchy(anb_ctx* c, int level, int array, long long* count, double* out) {
+  if (!c || !count) return ANB_ERR_INVALID;
+  return guarded(c, [&]() -> int {
+    const AmgDev& A = c->amg;
+    const bool last = level == A.nLevels - 1;
+    if (c->mixed || !c->amgBuilt || !A.sa || level < 0 || level >= A.nLevels || array < ANB_AMG_SIZES ||
+        array > ANB_AMG_R_VAL || (last && array >= ANB_AMG_AGG))
+      throw AnbError(ANB_ERR_INVALID, "no such array of a smoothed-aggregation hierarchy");
+    CK(cudaSetDevice(c->prm.device));
+    const AmgLevelDev& f = A.lv[level];
+    auto get = [&](auto* d, size_t n) {
+      std::vector<std::remove_const_t<std::remove_pointer_t<decltype(d)>>> h(n);
+      if (n) CK(cudaMemcpyAsync(h.data(), d, n * sizeof(h[0]), cudaMemcpyDeviceToHost, c->stream));
+      CK(cudaStreamSynchronize(c->stream));
+      return std::vector<double>(h.begin(), h.end());
+    };
+    auto end = [&](const int* off, int rows) { return (size_t)get(off + rows, 1)[0]; };
+    std::vector<double> v;
+    if (array == ANB_AMG_SIZES) {
+      v = {(double)A.nLevels, (double)f.n, (double)f.nc, (double)f.capQ, (double)f.capC};
+    } else if (array <= ANB_AMG_VAL && level == 0) {  // SELL-32
+      std::vector<double> off(1, 0.0), val = get(f.val, c->nEnt);
+      for (int r = 0; r < f.n; ++r) {
+        off.push_back(off.back() + c->L.rowLen[r]);
+        for (int k = 0; k < c->L.rowLen[r] && array != ANB_AMG_OFF; ++k) {
+          const int e = c->L.sliceOff[r / kSlice] + k * kSlice + r % kSlice;
+          v.push_back(array == ANB_AMG_COL ? c->L.col[e] : val[e]);
+        }
+      }
+      if (array == ANB_AMG_OFF) v = off;
+    } else {
+      switch (array) {
+        case ANB_AMG_OFF: v = get(f.rowOff, (size_t)f.n + 1); break;
+        case ANB_AMG_COL: v = get(f.col, end(f.rowOff, f.n)); break;
+        case ANB_AMG_VAL: v = get(f.val, end(f.rowOff, f.n)); break;
+        case ANB_AMG_DIAG: v = get(f.diag, f.n); break;
+        case ANB_AMG_WEIGHT: v = get(f.wdinv, f.n); break;
+        case ANB_AMG_AGG: v = get(f.agg, f.n); break;
+        case ANB_AMG_P_OFF: v = get(f.pOff, (size_t)f.n + 1); break;
+        case ANB_AMG_P_COL: v = get(f.pCol, end(f.pOff, f.n)); break;
+        case ANB_AMG_P_VAL: v = get(f.pVal, end(f.pOff, f.n)); break;
+        case ANB_AMG_Q_OFF: v = get(f.qOff, (size_t)f.n + 1); break;
+        case ANB_AMG_Q_COL: v = get(f.qCol, end(f.qOff, f.n)); break;
+        case ANB_AMG_R_OFF: v = get(f.tOff, (size_t)f.nc + 1); break;
+        case ANB_AMG_R_COL: v = get(f.tCol, f.nT); break;
+        default: v = get(f.tVal, f.nT); break;
+      }
+    }
+    *count = (long long)v.size();
+    if (out) std::copy(v.begin(), v.end(), out);
+    return ANB_OK;
+  });
+}
+
 }  // extern "C"
 
 namespace anb {

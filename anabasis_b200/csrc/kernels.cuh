@@ -345,7 +345,7 @@ struct AmgLevelDevT {
   int nEntNext;        // next level's SELL storage entries
   // work vectors
   T *b, *x, *x2;
-  T* wdinv;            // omega / diag (Jacobi smoother)
+  T* wdinv;            // Jacobi weights: omega / diag, bounded on the levels of kernels_sa.cu
   int maxW;            // level 0: largest SELL slice width
   // smoothed-aggregation hierarchies (AmgDevT::sa) only.  P by rows; A P by rows (the pattern of Q) and
   // Q = (I - w D^-1 A) P, whose values on level 0 are SELL-32 (qSlice, qColS: thread per row) and
@@ -408,6 +408,7 @@ void amg_dense_factor(const LaunchCfg& lc, const AmgLevelDevT<T>& c, double* inv
 // Smoothed-aggregation counterparts (kernels_sa.cu): values of one level step (P, Q, restriction and
 // the next level's matrix), all of them with the dense inverse, and the V-cycle of the PCG (mode 0).
 constexpr double kSaOmegaP = 2.0 / 3.0;
+constexpr double kSaWeight = 1.99;  // bound of w sum_j |a_ij| on the coarse levels
 template <class T>
 void sa_refresh_level(const LaunchCfg& lc, AmgDevT<T>& amg, int l);
 template <class T>

@@ -1,13 +1,19 @@
 // Smoothed-aggregation V(1,1)-cycle of the pressure CG and the refresh of its values (sm_100a),
 // standing in for the reference's BoomerAMG (main.cu:2224-2273).
 //
-// With one weighted-Jacobi sweep (weights w = omega / D) before and after the coarse correction,
-// the cycle of a level is
+// With one weighted-Jacobi sweep before and after the coarse correction, the cycle of a level is
 //   M^-1 b = w (b + r1) + Q A_c^-1 P^T r1,   r1 = b - A w b,   Q = (I - w A) P,   P^T r1 = Q^T b:
 // the post-smoothing is part of Q, which is stored, so no second product with A is needed.  Level 0
 // computes r1 (fused with the update of the PCG iteration) and restricts it with P^T (3.6 entries a
 // row on hexes against 8.6 of Q); the coarser levels, where a launch costs more than the bytes,
 // restrict b with Q^T and compute r1 in the up sweep: two launches a level.
+//
+// The weights are w = omega / a_ii on the finest level, whose rows are diagonally dominant.  The coarse
+// matrices have positive off-diagonals too and no such bound (the largest eigenvalue of D^-1 A reaches 2.4
+// where the coefficients spread over 1e6), so there w = min(omega / a_ii, 1.99 / sum_j |a_ij|): the matrix
+// of row sums minus A is positive semidefinite, hence w A < 2 and the cycle stays positive definite
+// whatever the coefficients.  Where the bound does not bind the weights are those of omega alone;
+// on isotropic grids the iterations are the same.
 //
 // Against the plain aggregation with over-correction (kernels_krylov.cu) the CG needs half the
 // iterations (143 -> 66 per SIMPLE step on 970k hexes, 151 -> 80 on 334k tets, both to 1e-15) with
@@ -117,10 +123,10 @@ __global__ void __launch_bounds__(kBlock) k_sa_restrict_block(const int* done, c
 }
 
 // Up sweep of a coarse level: out = x + w r1 + Q e with x = w b and r1 = b - A x, i.e.
-// (2 - omega) x_i + sum of the row [-w_i A_offdiag | Q] times [x | e].  The two matrices are stored as
+// (2 - w_i a_ii) x_i + sum of the row [-w_i A_offdiag | Q] times [x | e].  The two matrices are stored as
 // one CSR and the two vectors as one array, so a row is a single gather sum; G lanes a row.
 template <int G, class T>
-__global__ void __launch_bounds__(kBlock) k_sa_up(const int* done, AmgLevelDevT<T> f, double omega, T* out) {
+__global__ void __launch_bounds__(kBlock) k_sa_up(const int* done, AmgLevelDevT<T> f, T* out) {
   if (*done) return;
   const int lane = threadIdx.x & 31, sub = lane % G;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nWarps = (gridDim.x * blockDim.x) >> 5;
@@ -128,12 +134,13 @@ __global__ void __launch_bounds__(kBlock) k_sa_up(const int* done, AmgLevelDevT<
     const int i = base + lane / G;
     double y = 0.0;
     if (i < f.n) {
+      if (sub == 0) y = (2.0 - ld(&f.wdinv[i]) * ld(&f.diag[i])) * ld(&f.x[i]);
       const int k1 = __ldg(&f.mOff[i + 1]);
 #pragma unroll 8
       for (int k = __ldg(&f.mOff[i]) + sub; k < k1; k += G) y += ld(&f.mVal[k]) * ld(&f.x[__ldg(&f.mCol[k])]);
     }
     y = group_sum<G>(y);
-    if (i < f.n && sub == 0) out[i] = (T)((2.0 - omega) * ld(&f.x[i]) + y);
+    if (i < f.n && sub == 0) out[i] = (T)y;
   }
 }
 
@@ -201,7 +208,6 @@ struct SaTailArgs {
   int nLev;
   AmgLevelDevT<T> lv[kTailMaxLevels];
   const double* dense;
-  double omega;
 };
 
 // Rows of the cluster's CTAs in turn, a team of TS threads of one CTA a row.
@@ -239,19 +245,20 @@ __device__ __forceinline__ void tail_restrict(const AmgLevelDevT<T>& f, const Am
 }
 
 template <int G, class T>
-__device__ __forceinline__ void tail_up(const AmgLevelDevT<T>& f, double omega, int warp, int nWarps) {
+__device__ __forceinline__ void tail_up(const AmgLevelDevT<T>& f, int warp, int nWarps) {
   const int lane = threadIdx.x & 31, sub = lane % G;
   for (int base = warp * (32 / G); base < f.n; base += nWarps * (32 / G)) {
     const int i = base + lane / G;
     double y = 0.0;
     if (i < f.n) {
+      if (sub == 0) y = (2.0 - ld(&f.wdinv[i]) * ld(&f.diag[i])) * (double)__ldcg(&f.x[i]);
       const int k1 = __ldg(&f.mOff[i + 1]);
 #pragma unroll 8
       for (int k = __ldg(&f.mOff[i]) + sub; k < k1; k += G)
         y += ld(&f.mVal[k]) * (double)__ldcg(&f.x[__ldg(&f.mCol[k])]);
     }
     y = group_sum<G>(y);
-    if (i < f.n && sub == 0) f.x2[i] = (T)((2.0 - omega) * (double)__ldcg(&f.x[i]) + y);
+    if (i < f.n && sub == 0) f.x2[i] = (T)y;
   }
 }
 
@@ -281,8 +288,8 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_sa_tail(const int* done, co
   }
   for (int l = L - 2; l >= 0; --l) {
     cl.sync();
-    if (a.lv[l].n > 32 * nCta) tail_up<16>(a.lv[l], a.omega, warp, nWarps);
-    else tail_up<32>(a.lv[l], a.omega, warp, nWarps);
+    if (a.lv[l].n > 32 * nCta) tail_up<16>(a.lv[l], warp, nWarps);
+    else tail_up<32>(a.lv[l], warp, nWarps);
   }
 }
 
@@ -425,10 +432,12 @@ __global__ void __launch_bounds__(kBlock) k_sa_product(AmgLevelDevT<T> f, AmgLev
   }
   sync();
   if (!live) return;
+  double size = 0.0, diag = 0.0;  // sum of |a| over the row; the diagonal in the thread that has it
   for (int s = tt; s < nc + (kAP ? 0 : 1); s += TS) {
     double sum = 0.0;
 #pragma unroll 4
     for (int g = 0; g < NG; ++g) sum += acc[g * cap + s];
+    size += fabs(sum);
     if (kAP) {
       f.apVal[c0 + s] = (T)sum;
       const int J = cols[s];
@@ -442,8 +451,22 @@ __global__ void __launch_bounds__(kBlock) k_sa_product(AmgLevelDevT<T> f, AmgLev
       c.val[c0 + s] = (T)sum;
     } else {
       c.diag[r] = (T)sum;
-      c.wdinv[r] = (T)(omega / sum);
+      diag = sum;
     }
+  }
+  if constexpr (!kAP) {
+    if constexpr (TS > 32) {
+      __shared__ double sm[TS / 32];
+      size = warp_sum(size);
+      if ((tt & 31) == 0) sm[tt >> 5] = size;
+      __syncthreads();
+      size = 0.0;
+#pragma unroll
+      for (int u = 0; u < TS / 32; ++u) size += sm[u];
+    } else {
+      size = __shfl_sync(0xffffffffu, warp_sum(size), 0);
+    }
+    if (tt == nc % TS) c.wdinv[r] = (T)fmin(omega / diag, kSaWeight / size);
   }
 }
 
@@ -640,7 +663,6 @@ void sa_vcycle(const LaunchCfg& lc, const PcgArgsT<T>& a, const AmgDevT<T>* amg,
       ta.nLev = L - t0;
       for (int l = 0; l < ta.nLev; ++l) ta.lv[l] = amg->lv[t0 + l];
       ta.dense = amg->dense;
-      ta.omega = amg->omega;
       cudaLaunchAttribute at[1];
       const cudaLaunchConfig_t cfg = tail_config(lc.stream, amg->tailCluster, at);
       cudaLaunchKernelEx(&cfg, k_sa_tail<T>, (const int*)a.fl, ta);
@@ -651,8 +673,7 @@ void sa_vcycle(const LaunchCfg& lc, const PcgArgsT<T>& a, const AmgDevT<T>* amg,
     for (int l = t0 - 1; l >= 1; --l) {
       const AmgLevelDevT<T>& f = amg->lv[l];
       with_lanes(f.lanesUp, [&](auto G) {
-        k_sa_up<G.value, T><<<grid_for((long long)G.value * f.n, cap), kBlock, 0, lc.stream>>>(a.fl, f, amg->omega,
-                                                                                              f.x2);
+        k_sa_up<G.value, T><<<grid_for((long long)G.value * f.n, cap), kBlock, 0, lc.stream>>>(a.fl, f, f.x2);
       });
     }
   }

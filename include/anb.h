@@ -306,6 +306,26 @@ int anb_debug_nonorth(anb_ctx* ctx, const double* rau, const double* gx, const d
  * (p_tol, p_rel_tol); x holds the initial guess on entry.  *iters receives the count. */
 int anb_debug_pressure_solve(anb_ctx* ctx, const double* b, double* x, int* iters, double* final_res);
 
+/* One array of a level of the smoothed-aggregation hierarchy that is in place (FP64 contexts; after an
+ * iteration or anb_debug_pressure_solve), in the library's row numbering.  *count receives the length;
+ * out, when not NULL, the entries as doubles.  ANB_ERR_INVALID: no such hierarchy, level or array. */
+#define ANB_AMG_SIZES 0  /* levels, rows, rows of the next level, longest row of Q, of the next matrix + 1 */
+#define ANB_AMG_OFF 1    /* off-diagonals of the level's matrix by rows: offsets, columns, values */
+#define ANB_AMG_COL 2
+#define ANB_AMG_VAL 3
+#define ANB_AMG_DIAG 4
+#define ANB_AMG_WEIGHT 5 /* smoother */
+#define ANB_AMG_AGG 6    /* aggregate of every row */
+#define ANB_AMG_P_OFF 7  /* prolongator by rows */
+#define ANB_AMG_P_COL 8
+#define ANB_AMG_P_VAL 9
+#define ANB_AMG_Q_OFF 10 /* pattern of A P by rows */
+#define ANB_AMG_Q_COL 11
+#define ANB_AMG_R_OFF 12 /* restriction by coarse rows: P^T on the finest level, Q^T below */
+#define ANB_AMG_R_COL 13
+#define ANB_AMG_R_VAL 14
+int anb_debug_hierarchy(anb_ctx* ctx, int level, int array, long long* count, double* out);
+
 #ifdef __cplusplus
 }
 #endif
