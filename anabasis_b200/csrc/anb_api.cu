@@ -510,7 +510,7 @@ bool sa_pattern_device(anb_ctx* c, DevArena& ar, SaDevPattern& p, bool wantQT) {
 
 // The same from the host (sa_setup.cpp), uploaded.
 void sa_pattern_host(DevArena& ar, const SaMatrix& M, const std::vector<int>& agg, SaDevPattern& p, bool wantQT) {
-  const SaPattern S = sa_pattern(M, agg, p.nc, wantQT);
+  const SaPattern S = sa_pattern(M, agg, p.nc, wantQT, p.smooth);
   p.pOff = ar.upload(S.pOff);
   p.pCol = ar.upload(S.pCol);
   p.qOff = ar.upload(S.qOff);
@@ -535,7 +535,7 @@ void sa_pattern_host(DevArena& ar, const SaMatrix& M, const std::vector<int>& ag
 
 // Smoothed-aggregation hierarchy of the current level-0 matrix: aggregates on the host, patterns, values level
 // by level on the device (the next level's strong couplings come from them).  Returns false, with
-// nothing kept, when the coarsening stalls above the dense solver's size.
+// nothing kept, when a level step is refused (sa_coarsen).
 template <class T>
 bool build_sa(anb_ctx* c, AmgDevT<T>& A, DevArena& ar, T* val0, T* diag0, T* wdinv0, std::vector<double>& hv,
               std::vector<double>& hd) {
@@ -565,30 +565,28 @@ bool build_sa(anb_ctx* c, AmgDevT<T>& A, DevArena& ar, T* val0, T* diag0, T* wdi
   d->x2 = ar.alloc<T>(M.n);
   while (M.n > kDenseRows || l == 0) {
     if (l + 1 >= kSaMaxLevels) return reset(false);
-    // Where the next matrix would grow dense (or have a row too long for a block's shared memory),
-    // half the threshold is tried: fewer weak couplings, larger aggregates.
-    double theta = sa_theta(l, M.n, c->L.maxRowLen);
     SaDevPattern p;
-    int nc = 0;
+    SaStep step;
     AmgLevelDevT<T>& f = A.lv[l];
-    for (int tries = 0;; ++tries, theta *= 0.5) {
-      const std::vector<int> agg = sa_aggregate(M, theta, nc);
-      if (nc < 1 || nc > (int)(0.9 * M.n)) return reset(false);
-      if (tries < 3 && sa_next_entries(M, agg, nc) > 1.25 * M.col.size()) continue;
+    for (bool groups = false;; groups = true) {
+      if (!sa_coarsen(M, l, c->L.maxRowLen, groups, step)) return reset(false);
       p = SaDevPattern{};
       p.n = M.n;
-      p.nc = nc;
+      p.nc = step.nc;
+      p.smooth = step.smooth;
       p.sliceOff = f.sliceOff;
       p.rowOff = f.rowOff;
       p.col = f.col;
-      p.agg = ar.upload(agg);
-      if (!sa_pattern_device(c, ar, p, l > 0)) sa_pattern_host(ar, M, agg, p, l > 0);
+      p.agg = ar.upload(step.agg);
+      if (!sa_pattern_device(c, ar, p, l > 0)) sa_pattern_host(ar, M, step.agg, p, l > 0);
       if (sa_product_smem(8, 256, std::max(p.capQ, p.capC)) <= kSaSmemMax) break;
-      if (tries == 3) return reset(false);
+      if (!step.smooth) return reset(false);  // a row too long for a block's shared memory, grouped as well
     }
+    const int nc = step.nc;
     AmgLevelDevT<T>& k = A.lv[l + 1];
     k = AmgLevelDevT<T>{};
     f.nc = nc;
+    f.omegaP = step.smooth ? kSaOmegaP : 0.0;
     f.capQ = p.capQ;
     f.capC = p.capC;
     f.agg = p.agg;
@@ -689,7 +687,8 @@ void build_amg(anb_ctx* c, AmgDevT<T>& A, std::vector<AmgLevelHost>& H, DevArena
     hdd.assign(hd.begin(), hd.end());
   }
   const char* noGraph = std::getenv("ANB_NO_GRAPH");
-  if (ga && build_sa(c, A, ar, val0, diag0, wdinv0, hvd, hdd)) {
+  const char* smoothed = std::getenv("ANB_AMG_SMOOTHED");
+  if (ga && !(smoothed && smoothed[0] == '0') && build_sa(c, A, ar, val0, diag0, wdinv0, hvd, hdd)) {
     H.clear();
     c->amgBuilt = true;
     sa_configure_tail(A, kSaTailRows, c->stream);

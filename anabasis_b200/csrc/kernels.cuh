@@ -355,6 +355,7 @@ struct AmgLevelDevT {
   const int *pOff, *pCol, *qOff, *qCol, *qSlice, *qColS, *tOff, *tCol, *tSrc, *ptOff, *ptCol, *ptSrc,
       *mOff, *mCol;
   T *pVal, *apVal, *qVal, *tVal, *mVal;
+  double omegaP;       // P = (I - omegaP D^-1 A) P0: kSaOmegaP, or 0 where P is piecewise constant
   int nT;              // entries of the restriction operator
   int lanesDown, lanesUp;  // lanes per row of the restriction from (over 32: a block) and the up sweep of this level
   int capQ, capC;      // longest row of Q, and of the next level's matrix + 1
@@ -428,6 +429,7 @@ struct SaDevPattern {
   int n = 0, nc = 0;
   const int *sliceOff = nullptr, *rowOff = nullptr, *col = nullptr;  // the level's matrix (SELL-32 or CSR)
   const int* agg = nullptr;
+  bool smooth = true;  // P reaches the neighbours' aggregates
   int *pOff = nullptr, *pCol = nullptr, *qOff = nullptr, *qCol = nullptr, *cOff = nullptr, *cCol = nullptr;
   int *ptOff = nullptr, *ptCol = nullptr, *ptSrc = nullptr, *qtOff = nullptr, *qtCol = nullptr, *qtSrc = nullptr;
   int nP = 0, nQ = 0, nC = 0, capQ = 0, capC = 0;  // entries; longest rows of Q and of the next matrix

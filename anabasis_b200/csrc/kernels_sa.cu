@@ -326,9 +326,9 @@ __device__ __forceinline__ void row_entries(const AmgLevelDevT<T>& f, int i, int
 }
 
 // P = (I - omegaP D^-1 A) P0: G lanes a row, which sum each entry of P over the row's matrix entries
-// in turn (padding slots hold value 0).
+// in turn (padding slots hold value 0).  With omegaP = 0 the only entry, of the own aggregate, is 1.
 template <int G, class T>
-__global__ void __launch_bounds__(kBlock) k_sa_p(AmgLevelDevT<T> f, double omegaP) {
+__global__ void __launch_bounds__(kBlock) k_sa_p(AmgLevelDevT<T> f) {
   const int lane = threadIdx.x & 31, sub = lane % G;
   const int base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (32 / G);
   const int i = base + lane / G;
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(kBlock) k_sa_p(AmgLevelDevT<T> f, double omega
     k0 = __ldg(&f.pOff[i]);
     nk = __ldg(&f.pOff[i + 1]) - k0;
   }
-  const double s = d != 0.0 ? omegaP / d : 0.0;
+  const double s = d != 0.0 ? f.omegaP / d : 0.0;
   int most = nk;  // the rows of a warp run the same number of sums: group_sum needs every lane
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
@@ -596,9 +596,9 @@ void sa_refresh_level(const LaunchCfg& lc, AmgDevT<T>& amg, int l) {
   AmgLevelDevT<T>& f = amg.lv[l];
   AmgLevelDevT<T>& c = amg.lv[l + 1];
   g_launches += 4;
-  if (l == 0) k_sa_p<1, T><<<(f.n + kBlock - 1) / kBlock, kBlock, 0, lc.stream>>>(f, kSaOmegaP);
+  if (l == 0) k_sa_p<1, T><<<(f.n + kBlock - 1) / kBlock, kBlock, 0, lc.stream>>>(f);
   else with_lanes(f.lanesUp, [&](auto G) {
-    k_sa_p<G.value, T><<<grid_for((long long)G.value * f.n, 1 << 30), kBlock, 0, lc.stream>>>(f, kSaOmegaP);
+    k_sa_p<G.value, T><<<grid_for((long long)G.value * f.n, 1 << 30), kBlock, 0, lc.stream>>>(f);
   });
   refresh_q(lc, amg, l);
   k_sa_gather<T><<<grid_for(f.nT, 1 << 30), kBlock, 0, lc.stream>>>(f.nT, f.tSrc, l == 0 ? f.pVal : f.mVal, f.tVal);

@@ -18,6 +18,7 @@ struct PatTerm {  // rows of the product and their terms
   int rows;
   const int *sliceOff, *rowOff, *col;  // matrix pattern (SELL-32 or CSR): modes 0, 1
   const int* agg;
+  int smooth;                          // mode 0: with the neighbours
   const int *bOff, *bCol;              // rows of B: P (mode 1), A P (mode 2)
   const int *tOff, *tCol;              // P^T: mode 2
 };
@@ -70,6 +71,7 @@ __global__ void __launch_bounds__(kBlock) k_pattern(PatTerm a, int H, int* cnt, 
         n = a.rowOff[row + 1] - b;
         st = 1;
       }
+      if (MODE == 0 && !a.smooth) n = 0;
       for (int e = tt - 1; e < n; e += TS) {  // term -1: the row itself
         const int j = e < 0 ? row : a.col[b + e * st];
         if constexpr (MODE == 0) {
@@ -212,6 +214,7 @@ void sa_pattern_rows(const LaunchCfg& lc, const SaDevPattern& p, int mode, bool 
   a.rowOff = p.rowOff;
   a.col = p.col;
   a.agg = p.agg;
+  a.smooth = p.smooth;
   a.bOff = mode == 1 ? p.pOff : p.qOff;
   a.bCol = mode == 1 ? p.pCol : p.qCol;
   a.tOff = p.ptOff;

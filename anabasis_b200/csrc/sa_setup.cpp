@@ -80,6 +80,17 @@ void transpose(int n, int nc, const std::vector<int>& off, const std::vector<int
   }
 }
 
+// Aggregates numbered by their first row.
+std::vector<int> renumber(std::vector<int> agg, int nc) {
+  std::vector<int> ren(nc, -1);
+  int next = 0;
+  for (int& a : agg) {
+    if (ren[a] < 0) ren[a] = next++;
+    a = ren[a];
+  }
+  return agg;
+}
+
 }  // namespace
 
 std::vector<int> sa_aggregate(const SaMatrix& A, double theta, int& nc) {
@@ -124,13 +135,7 @@ std::vector<int> sa_aggregate(const SaMatrix& A, double theta, int& nc) {
       if (agg[A.col[k]] < 0 && strong(i, k)) agg[A.col[k]] = nc;
     ++nc;
   }
-  std::vector<int> ren(nc, -1);
-  int next = 0;
-  for (int i = 0; i < n; ++i) {
-    if (ren[agg[i]] < 0) ren[agg[i]] = next++;
-    agg[i] = ren[agg[i]];
-  }
-  return agg;
+  return renumber(std::move(agg), nc);
 }
 
 double sa_next_entries(const SaMatrix& A, const std::vector<int>& agg, int nc) {
@@ -178,7 +183,61 @@ double sa_next_entries(const SaMatrix& A, const std::vector<int>& agg, int nc) {
   return (double)sum / rows * nc;
 }
 
-SaPattern sa_pattern(const SaMatrix& A, std::vector<int> aggIn, int nc, bool wantQT) {
+std::vector<int> sa_groups(const SaMatrix& A, int size, int& nc) {
+  const int n = A.n;
+  // strength |a_ij| / sqrt(a_ii a_jj), squared and without the row's own factor
+  auto strength = [&](int k) { return A.val[k] < 0.0 ? A.val[k] * A.val[k] / A.diag[A.col[k]] : 0.0; };
+  std::vector<int> agg(n, -1);
+  std::vector<std::pair<double, int>> near;
+  nc = 0;
+  for (int i = 0; i < n; ++i) {
+    if (agg[i] >= 0) continue;
+    near.clear();
+    for (int k = A.off[i]; k < A.off[i + 1]; ++k)
+      if (agg[A.col[k]] < 0 && strength(k) > 0.0) near.push_back({strength(k), A.col[k]});
+    if (near.empty()) continue;
+    const size_t m = std::min(near.size(), (size_t)size - 1);
+    std::partial_sort(near.begin(), near.begin() + m, near.end(), [](const auto& x, const auto& y) {
+      return x.first != y.first ? x.first > y.first : x.second < y.second;
+    });
+    agg[i] = nc;
+    for (size_t q = 0; q < m; ++q) agg[near[q].second] = nc;
+    ++nc;
+  }
+  std::vector<int> join(agg);
+  for (int i = 0; i < n; ++i) {
+    if (agg[i] >= 0) continue;
+    double best = 0.0;
+    for (int k = A.off[i]; k < A.off[i + 1]; ++k)
+      if (agg[A.col[k]] >= 0 && strength(k) > best) {
+        best = strength(k);
+        join[i] = agg[A.col[k]];
+      }
+    if (join[i] < 0) join[i] = nc++;
+  }
+  return renumber(std::move(join), nc);
+}
+
+bool sa_coarsen(const SaMatrix& A, int level, int maxRowLen, bool groups, SaStep& step) {
+  step = SaStep{};
+  if (!groups) {
+    const double most = 1.25 * (double)A.col.size();
+    double theta = sa_theta(level, A.n, maxRowLen), next = 0.0;
+    for (int left = 3;; --left, theta *= 0.5) {
+      step.agg = sa_aggregate(A, theta, step.nc);
+      next = sa_next_entries(A, step.agg, step.nc);
+      if (left == 0 || next <= most || (level == 0 && theta < 2 * kSaLeastTheta)) break;
+    }
+    const bool slow = step.nc > A.n / 2, dense = level > 0 ? next > most : A.n > kSaDenseRows && next > 10.0 * A.n;
+    if (!slow && !dense) return true;
+  }
+  if (!sa_groupable(A, level)) return false;
+  step.smooth = false;
+  step.agg = sa_groups(A, kSaGroupSize, step.nc);
+  return step.nc <= A.n / 2;
+}
+
+SaPattern sa_pattern(const SaMatrix& A, std::vector<int> aggIn, int nc, bool wantQT, bool smooth) {
   SaPattern S;
   S.n = A.n;
   S.nc = nc;
@@ -191,7 +250,7 @@ SaPattern sa_pattern(const SaMatrix& A, std::vector<int> aggIn, int nc, bool wan
       out.push_back(I);
     };
     add(S.agg[i]);
-    for (int k = A.off[i]; k < A.off[i + 1]; ++k) add(S.agg[A.col[k]]);
+    for (int k = A.off[i]; smooth && k < A.off[i + 1]; ++k) add(S.agg[A.col[k]]);
   });
   build_rows(n, nc, S.qOff, S.qCol, [&](int i, std::vector<int>& out, std::vector<int>& mark) {
     auto add = [&](int j) {

@@ -47,8 +47,41 @@ inline double sa_theta(int level, int n, int maxRowLen) {
 std::vector<int> sa_aggregate(const SaMatrix& A, double theta, int& nc);
 // Estimate of the next matrix's off-diagonal entries for these aggregates, from every 16th of its rows.
 double sa_next_entries(const SaMatrix& A, const std::vector<int>& agg, int nc);
-// All patterns of one level step for the given aggregates.
-SaPattern sa_pattern(const SaMatrix& A, std::vector<int> agg, int nc, bool wantQT);
+// Aggregates of up to `size` rows, each a row with its strongest free neighbours (rows left over join their
+// strongest neighbour's), whatever the threshold: a full matrix shrinks by about that factor.
+std::vector<int> sa_groups(const SaMatrix& A, int size, int& nc);
+
+// One level step.  The threshold is halved, at most three times, while the next matrix would hold more than
+// 1.25 times this one's entries: fewer weak couplings, larger aggregates.  It is the first sign of trouble
+// when that does not help, or when less than half of the rows go (weak couplings throughout: spread
+// coefficients, or a level that is nearly full).  Then
+//  - a deep level (the third of the hierarchy or lower, up to kSaGroupRows rows) or a second one that is a
+//    quarter full is grouped by eight with a piecewise constant P (smooth = false): the next matrix has no
+//    more entries a row than this one;
+//  - otherwise the step is refused, and the plain aggregation serves, before another level has been built.
+// On the finest level the threshold stays at kSaLeastTheta or more, which keeps the weak directions of a
+// stretched grid weak.  Flat cells (two weak directions) are then joined to lines of three and the second level
+// is dense, 16 entries for every finest row of a hex grid and 8 on tets.  It coarsens well again up to 16:1,
+// and pays where launches set the time of a cycle: ms a step, taken / refused, 36k hexes of 10:1 3.1 / 5.4,
+// 97k 5.2 / 6.3, 246k 9.2 / 10.0, 980k 39.4 / 23.8; 691k tets 19.5 / 28.2.  It is refused above kSaDenseRows
+// rows with more than 10 entries for each.  groups: go to the groups at once (the caller found a row too
+// long for the device's products).
+struct SaStep {
+  std::vector<int> agg;
+  int nc = 0;
+  bool smooth = true;
+};
+constexpr double kSaLeastTheta = 0.01;
+constexpr int kSaDenseRows = 250000;
+constexpr int kSaGroupRows = 16384;
+constexpr int kSaGroupSize = 8;
+inline bool sa_groupable(const SaMatrix& A, int level) {
+  return level > 1 ? A.n <= kSaGroupRows : level == 1 && 4.0 * A.col.size() > (double)A.n * A.n;
+}
+bool sa_coarsen(const SaMatrix& A, int level, int maxRowLen, bool groups, SaStep& step);
+
+// All patterns of one level step for the given aggregates; P is piecewise constant without smooth.
+SaPattern sa_pattern(const SaMatrix& A, std::vector<int> agg, int nc, bool wantQT, bool smooth = true);
 // The level-0 matrix as CSR; vals in the layout's SELL-32 storage.
 SaMatrix sa_fine_matrix(const Layout& L, const std::vector<double>& vals, const std::vector<double>& diag);
 
