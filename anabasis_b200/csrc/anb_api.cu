@@ -1335,6 +1335,10 @@ int anb_create(const anb_mesh_desc* md, const anb_params* prm, anb_ctx** out) {
     c->ab.nnzOff = 2LL * c->nI;
 
     DevArena& A = c->arena;
+    // bytes a cell of a hex grid (the boundary's share apart) with little to spare
+    A.expect((size_t)1500 * c->C + (size_t)400 * c->nB);
+    c->scalarArena.expect((size_t)220 * c->C + (size_t)40 * c->nB);
+    c->amgArena.expect((size_t)1000 * c->C);
     // faces
     std::vector<FaceRec> fr(c->nI);
     for (int f = 0; f < c->nI; ++f) {

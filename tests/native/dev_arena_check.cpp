@@ -96,6 +96,28 @@ int main() {
   anb::build_once(ready, a, make);
   if (first != was) return fail("a ready group was made twice");
   a.release();
+
+  // a context's requests, from a few bytes to a share of a large grid: little is held beyond them, and another
+  // round of them in another order and a per cent smaller takes no more memory
+  for (size_t cells : {(size_t)2000, (size_t)50000, (size_t)1000000}) {
+    anb::DevArena b;
+    b.expect(1300 * cells);
+    size_t asked = 0, calls = g_blocks.size();
+    const int per[] = {192, 4, 64, 24, 8, 8, 96, 1, 24, 53, 24, 8, 48, 512, 24, 24, 8, 8, 24, 24, 96, 24};
+    for (int p : per) asked += p * cells, b.alloc<char>(p * cells);
+    if (b.bytes() > asked * 1.1 + (3u << 20)) return fail("an arena holds far more than was asked for");
+    if (g_blocks.size() - calls > 2 + (cells > 20000 ? 22 : 0)) return fail("a small arena took many allocations");
+    const size_t held = g_held;
+    b.recycle();
+    for (int p : {512, 96, 96, 192, 64, 53, 48, 24, 24, 24, 24, 24, 24, 24, 8, 8, 8, 8, 4, 1})
+      b.alloc<char>(p * cells * 99 / 100);
+    if (b.bytes() <= anb::DevArena::kKeep && g_held > held) return fail("a recycled arena grew");
+    b.release();
+  }
+  a.alloc<char>(anb::DevArena::kKeep / 2 + 1);
+  a.alloc<char>(anb::DevArena::kKeep / 2 + 1);
+  a.recycle();
+  if (g_held) return fail("a large arena outlived its use");
   std::printf("ok\n");
   return 0;
 }
