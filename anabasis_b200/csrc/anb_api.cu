@@ -668,12 +668,21 @@ bool build_sa(anb_ctx* c, AmgDevT<T>& A, DevArena& ar, T* val0, T* diag0, T* wdi
   return true;
 }
 
+// Forgets a hierarchy that is half built.
+template <class T>
+void drop_hierarchy(anb_ctx* c, AmgDevT<T>& A, DevArena& ar) {
+  CK(cudaStreamSynchronize(c->stream));
+  ar.release();
+  A.nLevels = A.sa = 0;
+  A.dense = nullptr;
+}
+
 // Aggregation hierarchy for the current level-0 matrix (val0/diag0 on the device, storage type T),
 // coarse levels in T, coarsest inverse in double, host structure in H, device arrays in ar.  For the
 // pressure hierarchy (ga != nullptr) the PCG V-cycles are captured as graphs for *ga.
 template <class T>
-void build_amg(anb_ctx* c, AmgDevT<T>& A, std::vector<AmgLevelHost>& H, DevArena& ar, T* val0, T* diag0, T* wdinv0,
-               const PcgArgsT<T>* ga) {
+void build_levels(anb_ctx* c, AmgDevT<T>& A, std::vector<AmgLevelHost>& H, DevArena& ar, T* val0, T* diag0, T* wdinv0,
+                  const PcgArgsT<T>* ga) {
   std::vector<T> hv(c->nEnt), hd(c->C);
   CK(cudaMemcpyAsync(hv.data(), val0, hv.size() * sizeof(T), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaMemcpyAsync(hd.data(), diag0, hd.size() * sizeof(T), cudaMemcpyDeviceToHost, c->stream));
@@ -688,7 +697,15 @@ void build_amg(anb_ctx* c, AmgDevT<T>& A, std::vector<AmgLevelHost>& H, DevArena
   }
   const char* noGraph = std::getenv("ANB_NO_GRAPH");
   const char* smoothed = std::getenv("ANB_AMG_SMOOTHED");
-  if (ga && !(smoothed && smoothed[0] == '0') && build_sa(c, A, ar, val0, diag0, wdinv0, hvd, hdd)) {
+  bool sa = false;
+  if (ga && !(smoothed && smoothed[0] == '0')) {
+    try {
+      sa = build_sa(c, A, ar, val0, diag0, wdinv0, hvd, hdd);
+    } catch (const NoDeviceMemory&) {  // 700 bytes a cell on hexes, against 160 of the plain aggregation
+      drop_hierarchy(c, A, ar);
+    }
+  }
+  if (sa) {
     H.clear();
     c->amgBuilt = true;
     sa_configure_tail(A, kSaTailRows, c->stream);
@@ -770,6 +787,18 @@ void build_amg(anb_ctx* c, AmgDevT<T>& A, std::vector<AmgLevelHost>& H, DevArena
     std::fprintf(stderr, " | tail rows %d, cluster %d\n", A.tailRows, A.tailCluster);
   }
   if (ga && A.nLevels >= 2 && !(noGraph && noGraph[0] == '1')) CK(amg_capture_graph(c->lc, *ga, A));
+}
+
+template <class T>
+void build_amg(anb_ctx* c, AmgDevT<T>& A, std::vector<AmgLevelHost>& H, DevArena& ar, T* val0, T* diag0, T* wdinv0,
+               const PcgArgsT<T>* ga) {
+  try {
+    build_levels(c, A, H, ar, val0, diag0, wdinv0, ga);
+  } catch (const NoDeviceMemory&) {
+    drop_hierarchy(c, A, ar);
+    if (ga) c->amgBuilt = false;
+    throw;
+  }
 }
 
 // Momentum AMG (mom_amg): Jacobi weights of the freshly assembled matrix, the hierarchy on first

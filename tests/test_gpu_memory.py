@@ -1,8 +1,12 @@
-"""Device memory of contexts."""
+"""Device memory of contexts: small ones hold little, and a grid whose smoothed-aggregation hierarchy does not fit
+runs on the plain aggregation, which needs a quarter of its memory."""
+import os
+
 import numpy as np
 import pytest
 
 import anabasis_b200 as anb
+from tests.cases import channel, initial_state
 
 pytestmark = pytest.mark.gpu
 
@@ -29,3 +33,42 @@ def test_small_contexts_hold_little():
     held = [make() for _ in range(12)]
     assert before - _free() <= 12 * 14 * 2**20
     assert first.n_cells == held[0].n_cells
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_hierarchy_that_does_not_fit(precision):
+    import torch
+
+    m, bc, _ = channel(nx=110, ny=62, nz=60, jitter=0.1, seed=2)  # 409,200 cells: 290 MB smoothed, 65 MB plain (FP64)
+    init = initial_state(m, bc)
+    prm = dict(rho=1.0, mu=1e-3, u_relax=0.7, p_relax=0.3, precision=precision)
+
+    def solver():
+        s = anb.Solver(m, anb.default_params(**prm))
+        s.set_bc(bc)
+        s.set_state(*init)
+        return s
+
+    os.environ["ANB_AMG_SMOOTHED"] = "0"
+    try:
+        s = solver()
+        _, want = s.iterate(2)
+        fields = s.get_state()
+        s.close()
+    finally:
+        del os.environ["ANB_AMG_SMOOTHED"]
+    s = solver()  # its whole run once, so that every kernel is loaded
+    _, smoothed = s.iterate(1)
+    s.close()
+    s = solver()
+    room = 120 * 2**20  # between the two needs, FP32 storage included
+    filler = torch.empty(_free() - room, dtype=torch.uint8, device="cuda")
+    try:
+        rc, st = s.iterate(2)
+        got = s.get_state()
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    assert rc == anb.ANB_OK and smoothed[0]["its_p_total"] < want[0]["its_p_total"]
+    assert [x["its_p_total"] for x in st] == [x["its_p_total"] for x in want]
+    assert all(np.array_equal(got[k], fields[k]) for k in "uvwp")
