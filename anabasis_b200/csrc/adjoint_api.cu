@@ -251,8 +251,7 @@ void mom_solve(anb_ctx* c, AdjointData& d, bool trans, const double* b, double* 
   a.maxit = d.momMaxit;
   a.red = c->red;
   CK(cudaMemsetAsync(x, 0, sizeof(double) * 3 * c->C, c->stream));
-  const int fam = c->prof.family;  // a timed kernel family runs from the host loops
-  if (fam != kKfBicgSpmv && fam != kKfBicgVector && bicg_coop_solve(c->lc, a, 7, c->nSM, c->coopPart)) {
+  if (!bicg_timed(c) && bicg_coop_solve(c->lc, a, 7, c->nSM, c->coopPart)) {
     adj_count_prec(c->lc, a.fl, nullptr, d.cnt);  // read with the iteration's Hessenberg column
     return;
   }

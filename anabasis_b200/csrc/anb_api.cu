@@ -240,9 +240,7 @@ void mom_apply(void* ctx, int q, int which) {
 // with `out` given, on their way to out->slot.
 template <class T>
 int bicg_iterate(anb_ctx* c, const BicgArgsT<T>& a, BicgLoopT<T>& loop, SolveOut* out) {
-  const int fam = c->prof.family;
-  const bool timed = fam == kKfBicgSpmv || fam == kKfBicgVector;
-  if (!timed && bicg_loop_launch(c->lc, a, loop)) {
+  if (!bicg_timed(c) && bicg_loop_launch(c->lc, a, loop)) {
     if (out) {
       out->kernelsPerIteration = 5;
       out->slot = defer_flags(c, a.fl, 13);
@@ -295,8 +293,7 @@ void solve_momentum(anb_ctx* c, const int* active, SolveOut* out, bool defer) {
   a.maxit = c->prm.vel_maxit;
   a.red = c->red;
   a.precond = (c->prm.mom_amg && c->momAmgBuilt && c->amgMom.nLevels >= 2) ? 1 : 0;
-  const int fam = c->prof.family;
-  if (fam != kKfBicgSpmv && fam != kKfBicgVector &&
+  if (!bicg_timed(c) &&
       bicg_coop_solve(c->lc, a, active[0] | active[1] << 1 | active[2] << 2, c->nSM, c->coopPart)) {
     out->coop = true;
     if (defer) out->slot = defer_flags(c, a.fl, 14);
@@ -1929,7 +1926,7 @@ int anb_scalar_transport_solve(anb_ctx* c, const double* flux, const double* gam
       if (a.nonorth) launch_scalar_grad(c->lc, c->dm, a);
       launch_scalar_assemble(c->lc, c->dm, a);
       int done = 0;
-      if (bicg_coop_solve(c->lc, b, 1, c->nSM, c->coopPart)) {
+      if (!bicg_timed(c) && bicg_coop_solve(c->lc, b, 1, c->nSM, c->coopPart)) {
         poll(c, b.fl, 14);
         check_coop(c->hFlags);
         its = c->hFlags[2];

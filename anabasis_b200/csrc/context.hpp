@@ -174,6 +174,10 @@ DSell mom_sell(const anb_ctx* c);
 DSell p_sell(const anb_ctx* c);
 void grad(anb_ctx* c, int nf, const double* const* phi, const unsigned char* bits, double* const* out);
 void poll(anb_ctx* c, const int* dflags, int count);
+// A kernel family of the BiCGSTAB is being timed: its solves then run kernel by kernel from the host loops.
+inline bool bicg_timed(const anb_ctx* c) {
+  return c->prof.family == kKfBicgSpmv || c->prof.family == kKfBicgVector;
+}
 // Throws when the flags of a BiCGSTAB solve report a barrier that timed out (bicg_coop_solve).
 void check_coop(const int* flags);
 PcgArgs pcg_args(anb_ctx* c, const double* b, double rtol);
