@@ -433,7 +433,7 @@ PcgArgsT<float> pcg_args32(anb_ctx* c, const float* b, float* x, double atol, do
 // Coarse levels of at most this many rows run as one cluster kernel (ANB_AMG_TAIL_ROWS overrides;
 // 0 launches every level and sweep separately).  The arithmetic is the same either way.
 constexpr int kAmgTailRows = 1024;
-// The same for the smoothed-aggregation hierarchy.
+// The same for the smoothed-aggregation hierarchy (ANB_SA_TAIL_ROWS), whose tail sums a row in another order.
 constexpr int kSaTailRows = 1024;
 // CSR levels of at most this many rows run down sweep + restriction as one kernel
 // (ANB_AMG_FUSED_DOWN_ROWS overrides; 0 = off).  Same values either way.
@@ -705,7 +705,8 @@ void build_levels(anb_ctx* c, AmgDevT<T>& A, std::vector<AmgLevelHost>& H, DevAr
   if (sa) {
     H.clear();
     c->amgBuilt = true;
-    sa_configure_tail(A, kSaTailRows, c->stream);
+    const char* tailRows = std::getenv("ANB_SA_TAIL_ROWS");
+    sa_configure_tail(A, tailRows ? std::atoi(tailRows) : kSaTailRows, c->stream);
     if (!(noGraph && noGraph[0] == '1')) CK(amg_capture_graph(c->lc, *ga, A));
     return;
   }
