@@ -234,7 +234,6 @@ void prec_setup(anb_ctx* c, AdjointData& d) {
   d.precReady = true;
 }
 
-
 // x (3C) = M^{-1} b with M the momentum matrix (transpose when trans), from x = 0
 void mom_solve(anb_ctx* c, AdjointData& d, bool trans, const double* b, double* x) {
   BicgArgs a{};
@@ -289,11 +288,11 @@ void p_solve(anb_ctx* c, AdjointData& d, const double* b, double* x) {
   d.pIts += c->hFlags[1];
 }
 
-void scale(anb_ctx* c, AdjointData&, size_t n, const double* src, double s, double* dst) {
+void scale(anb_ctx* c, size_t n, const double* src, double s, double* dst) {
   vec_axpby(c->lc, n, s, src, 0.0, dst);
 }
 // y = a x + b y (n)
-void axpby(anb_ctx* c, AdjointData&, size_t n, double a, const double* x, double b, double* y) {
+void axpby(anb_ctx* c, size_t n, double a, const double* x, double b, double* y) {
   vec_axpby(c->lc, n, a, x, b, y);
 }
 
@@ -307,7 +306,7 @@ void precondition(anb_ctx* c, AdjointData& d, bool trans, const double* s, doubl
     mom_solve(c, d, false, s, zU);                                  // dU* = A^-1 s_U
     adj_div_u(c->lc, c->dm, rho, zU, d.t1);                         // D_U dU*
     CK(cudaMemcpyAsync(d.t2, s + 3 * (size_t)C, sizeof(double) * C, cudaMemcpyDeviceToDevice, c->stream));
-    axpby(c, d, C, -d.schur / rho, d.t1, d.schur / rho, d.t2);    // uRelax (s_c - D_U dU*) / rho
+    axpby(c, C, -d.schur / rho, d.t1, d.schur / rho, d.t2);    // uRelax (s_c - D_U dU*) / rho
     p_solve(c, d, d.t2, zp);                                        // dp
     GradArgs ga{};
     ga.nf = 1;
@@ -320,11 +319,11 @@ void precondition(anb_ctx* c, AdjointData& d, bool trans, const double* s, doubl
   } else {
     adj_grad_t(c->lc, c->dm, d.rau, fac, s, d.t3, 8u, d.t1);        // (Dinv G)^T s_U
     CK(cudaMemcpyAsync(d.t2, s + 3 * (size_t)C, sizeof(double) * C, cudaMemcpyDeviceToDevice, c->stream));
-    axpby(c, d, C, -d.schur / rho, d.t1, d.schur / rho, d.t2);    // uRelax (s_c - ...) / rho
+    axpby(c, C, -d.schur / rho, d.t1, d.schur / rho, d.t2);    // uRelax (s_c - ...) / rho
     p_solve(c, d, d.t2, zp);
     adj_div_u_t(c->lc, c->dm, rho, zp, d.t1);                       // D_U^T z_p
     CK(cudaMemcpyAsync(d.t2, s, sizeof(double) * 3 * C, cudaMemcpyDeviceToDevice, c->stream));
-    axpby(c, d, 3 * (size_t)C, -1.0, d.t1, 1.0, d.t2);              // s_U - D_U^T z_p
+    axpby(c, 3 * (size_t)C, -1.0, d.t1, 1.0, d.t2);              // s_U - D_U^T z_p
     mom_solve(c, d, true, d.t2, zU);                                // A^-T (...)
   }
 }
@@ -366,7 +365,7 @@ KrylovResult fgmres(anb_ctx* c, AdjointData& d, bool trans, const double* b, dou
       if (trans) vjp(c, d, x, d.t3);
       else jvp(c, d, x, d.dgZero, 0.0, d.t3);
       CK(cudaMemcpyAsync(r, b, sizeof(double) * N, cudaMemcpyDeviceToDevice, c->stream));
-      axpby(c, d, N, -1.0, d.t3, 1.0, r);
+      axpby(c, N, -1.0, d.t3, 1.0, r);
     }
     first = false;
     const double beta = norm(c, d, N, r);
@@ -375,7 +374,7 @@ KrylovResult fgmres(anb_ctx* c, AdjointData& d, bool trans, const double* b, dou
       kr.conv = true;
       break;
     }
-    scale(c, d, N, r, 1.0 / beta, r);
+    scale(c, N, r, 1.0 / beta, r);
     std::fill(gvec.begin(), gvec.end(), 0.0);
     gvec[0] = beta;
     int j = 0;
@@ -435,7 +434,7 @@ KrylovResult fgmres(anb_ctx* c, AdjointData& d, bool trans, const double* b, dou
       if (trans) vjp(c, d, x, d.t3);
       else jvp(c, d, x, d.dgZero, 0.0, d.t3);
       CK(cudaMemcpyAsync(d.t2, b, sizeof(double) * N, cudaMemcpyDeviceToDevice, c->stream));
-      axpby(c, d, N, -1.0, d.t3, 1.0, d.t2);
+      axpby(c, N, -1.0, d.t3, 1.0, d.t2);
       kr.res = norm(c, d, N, d.t2);
       if (kr.res <= 1.5 * target) {
         kr.conv = true;
@@ -613,12 +612,12 @@ int anb_newton_solve(anb_ctx* c, int maxNewton, double tol, int linMaxIt, int* s
       rn = norm(c, d, d.N, d.R);
       if (rn <= tol || k >= maxNewton) break;
       prec_setup(c, d);
-      scale(c, d, d.N, d.R, -1.0, d.rhs);
+      scale(c, d.N, d.R, -1.0, d.rhs);
       kr = fgmres(c, d, false, d.rhs, d.xs, 1e-3, linMaxIt);
       total += kr.its;
       // X += dX
-      axpby(c, d, 3 * (size_t)c->C, 1.0, d.xs, 1.0, c->U);
-      axpby(c, d, (size_t)c->C, 1.0, d.xs + 3 * (size_t)c->C, 1.0, c->P);
+      axpby(c, 3 * (size_t)c->C, 1.0, d.xs, 1.0, c->U);
+      axpby(c, (size_t)c->C, 1.0, d.xs + 3 * (size_t)c->C, 1.0, c->P);
     }
     if (steps) *steps = k;
     if (resNorm) *resNorm = rn;
@@ -643,7 +642,7 @@ int anb_tangent_linear(anb_ctx* c, int patch, int sign, const double dir[3], con
     upload_bc3(c, dbc, d.dgDir);
     CK(cudaMemsetAsync(d.t1, 0, sizeof(double) * d.N, c->stream));
     jvp(c, d, d.t1, d.dgDir, dmu, d.rhs);  // R_theta dtheta
-    scale(c, d, d.N, d.rhs, -1.0, d.rhs);
+    scale(c, d.N, d.rhs, -1.0, d.rhs);
     KrylovResult kr = fgmres(c, d, false, d.rhs, d.xs, d.rtol, 2000);
     adj_objective(c->lc, c->dm, adj_args(c, d), obj_args(c, d, patch, sign, dir), d.gX);
     vec_mdot(c->lc, d.N, 1, d.gX, d.N, d.xs, d.partials, d.coef);

@@ -11,6 +11,11 @@
 // (cooperative launch); a barrier that is not reached within kSpinLimit polls sets the fail flag and every
 // block returns.
 //
+// rho of the next step is rh.s - omega rh.t, whose sums are due with those of t, where the five kernels sum rh.r
+// of the new residual at a barrier of its own: a rounding of eps |rh| |s| in place of eps |rh| |r|, with |s| / |r|
+// one half step's reduction.  It enters beta alone, so the search directions and never the recurrences of x and r;
+// the iterations are the five kernels' to a few per cent.
+//
 // Measured (ms per pass, five kernels -> one): SIMPLE steps on 16k hexes 21.4 -> 15.5, 36k with all
 // correctors 22.9 -> 18.0, scalar transport on 262k cells 44 -> 24, force gradient at 36k 88 -> 70; with
 // the matrix of four rows a thread in shared memory instead of L2, and no fences beyond the release and

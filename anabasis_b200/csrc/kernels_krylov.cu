@@ -1441,7 +1441,6 @@ void amg_dense_factor(const LaunchCfg& lc, const AmgLevelDevT<T>& c, double* inv
   else go(k_amg_dense_factor<T, 5>);
 }
 
-
 template <class T>
 void amg_refresh(const LaunchCfg& lc, AmgDevT<T>& amg) {
   if (amg.sa) return sa_refresh(lc, amg);
