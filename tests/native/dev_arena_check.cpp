@@ -97,8 +97,8 @@ int main() {
   if (first != was) return fail("a ready group was made twice");
   a.release();
 
-  // a context's requests, from a few bytes to a share of a large grid: little is held beyond them, and another
-  // round of them in another order and a per cent smaller takes no more memory
+  // a context's requests, from a few bytes to a share of a large grid: little is held beyond them, and a second
+  // set of them in another order and a per cent smaller takes no more memory
   for (size_t cells : {(size_t)2000, (size_t)50000, (size_t)1000000}) {
     anb::DevArena b;
     b.expect(1300 * cells);
